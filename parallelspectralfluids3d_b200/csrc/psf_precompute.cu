@@ -4,15 +4,18 @@
 //   psf_csr_cheb     one warp per row of a CSR matrix, 16-byte gathers of the
 //                    block's rows, fused with the Chebyshev three-term
 //                    recurrence (out = alpha A Y + beta Y + gamma X)
-//   psf_wedge_w      W[e][kk][j] = sum_g q_e[g][kk] Phi[g_e][j] with
-//                    q_e[g][kk] = sum_f S_e[f][g] Phi[f_e][k0 + kk] over the
+//   psf_wedge_w      W[e][k][j] = sum_g q_e[g][k] Phi[g_e][j] with
+//                    q_e[g][k] = sum_f S_e[f][g] Phi[f_e][k] over the
 //                    (at most 8) faces the edge's terms name: the wedge
-//                    matrices of a batch of modes, one warp per edge
+//                    matrices of a batch of modes, one warp per edge.  S_e is
+//                    antisymmetric, so W[e][k][j] = -W[e][j][k] and only the
+//                    columns j > k of a mode are made
 //   psf_wedge_gemm   partial[s][a][c] = sum_{e in split s} Psi[e][a] W[e][c]:
-//                    a 128 x 128 x 16 FP64 tile GEMM with a three-stage
-//                    cp.async pipeline, split along the edges
-//   psf_wedge_reduce C[k][a][j] = (1/lambda_k) sum_s partial[s][a][kk ldn + j],
-//                    splits summed in a fixed order (deterministic)
+//                    a 64 x 128 x 16 FP64 tile GEMM on mma.sync with a
+//                    three-stage cp.async pipeline, split along the edges
+//   psf_wedge_reduce C[k][a][j] = (1/lambda_k) sum_s partial[s][a][(k, j)] and
+//                    C[j][a][k] = -(1/lambda_j) of the same sum, splits summed
+//                    in a fixed order (deterministic)
 //
 // The reference builds the same tensor with dense E x N matrices per mode
 // (Solver/SolverImpl/psfsolver.cpp:431-551); here the 12 wedge terms of every
@@ -112,12 +115,25 @@ __global__ void __launch_bounds__(256) psf_csr_cheb(long long n_rows, int m2, lo
 constexpr int WEDGE_KB_MAX = 64;  // modes per W batch (shared-memory q table)
 constexpr int SLOTS = PSF_WEDGE_SLOTS;
 
+// Columns of a batch of modes k0 .. k0 + kb: mode k has the columns j from
+// first_of(k) (k + 1 rounded down to even, for 16-byte accesses) to N rounded
+// up to even, one mode after the other.
+__host__ __device__ __forceinline__ int first_of(int k) { return (k + 1) & ~1; }
+__host__ __device__ __forceinline__ long long columns_before(int N, int k0, int k)
+{
+    // sum over k0 <= i < k of (N2 - first_of(i)); first_of sums to m (m + 1) / 2 rounded per parity
+    const long long N2 = (N + 1) & ~1;
+    const long long f1 = (long long)(k / 2) * ((k + 1) / 2), f0 = (long long)(k0 / 2) * ((k0 + 1) / 2);
+    return (long long)(k - k0) * N2 - 2 * (f1 - f0);
+}
+
 // One warp per edge: q_e[g][kk] in shared memory (used slots compacted to
 // the front), then the edge's W rows.  Slots holding the zero row are
 // skipped; the test is warp-uniform.  Rows e >= n_edges (padding up to whole
-// GEMM chunks) are written as zeros.
-__global__ void __launch_bounds__(256) psf_wedge_w(long long n_edges, long long n_rows, int ldn, int k0, int kb,
-                                                   const int32_t *__restrict__ edge_faces,
+// GEMM chunks) are written as zeros.  Bound by the stores: 0.18 ms for the
+// 0.72 GB of two batches at 16^3, N = 128 (0.28 ms with all columns).
+__global__ void __launch_bounds__(256) psf_wedge_w(long long n_edges, long long n_rows, int N, int ldn, long long ldc,
+                                                   int k0, int kb, const int32_t *__restrict__ edge_faces,
                                                    const double *__restrict__ edge_S,
                                                    const double *__restrict__ phi, long long zero_row,
                                                    double *__restrict__ W)
@@ -126,11 +142,11 @@ __global__ void __launch_bounds__(256) psf_wedge_w(long long n_edges, long long 
     __shared__ int32_t fs[8][SLOTS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long long nwarps = (long long)gridDim.x * 8;
-    const int ld2 = ldn / 2;
+    const int n2 = (N + 1) / 2;
     for (long long e = (long long)blockIdx.x * 8 + warp; e < n_rows; e += nwarps) {
-        double2 *We = reinterpret_cast<double2 *>(W + (size_t)e * kb * ldn);
+        double2 *We = reinterpret_cast<double2 *>(W + (size_t)e * ldc);
         if (e >= n_edges) {
-            for (int i = lane; i < kb * ld2; i += 32) We[i] = make_double2(0.0, 0.0);
+            for (long long i = lane; i < ldc / 2; i += 32) We[i] = make_double2(0.0, 0.0);
             continue;
         }
         __syncwarp();
@@ -160,12 +176,18 @@ __global__ void __launch_bounds__(256) psf_wedge_w(long long n_edges, long long 
                 ++used;
             }
         __syncwarp();
-        for (int j2 = lane; j2 < ld2; j2 += 32) {
+        for (int c2 = first_of(k0) / 2; c2 < n2; c2 += 32) {
+            const int j2 = c2 + lane;
             double2 p[SLOTS];
 #pragma unroll
             for (int g = 0; g < SLOTS; ++g)
-                if (g < used) p[g] = __ldg(reinterpret_cast<const double2 *>(phi + (size_t)fs[warp][g] * ldn) + j2);
-            for (int kk = 0; kk < kb; ++kk) {
+                if (g < used && j2 < n2)
+                    p[g] = __ldg(reinterpret_cast<const double2 *>(phi + (size_t)fs[warp][g] * ldn) + j2);
+            // Modes with a column in this run; `at` is the place of mode k's column pair 0.
+            const int kend = min(kb, 2 * min(c2 + 32, n2) - k0);
+            double2 *at = We - first_of(k0) / 2;
+            for (int kk = 0; kk < kend; ++kk) {
+                const int first2 = first_of(k0 + kk) / 2;
                 double2 w = make_double2(0.0, 0.0);
 #pragma unroll
                 for (int g = 0; g < SLOTS; ++g)
@@ -174,15 +196,18 @@ __global__ void __launch_bounds__(256) psf_wedge_w(long long n_edges, long long 
                         w.x = fma(q, p[g].x, w.x);
                         w.y = fma(q, p[g].y, w.y);
                     }
-                We[(size_t)kk * ld2 + j2] = w;
+                if (j2 >= first2 && j2 < n2) at[j2] = w;
+                at += n2 - first_of(k0 + kk + 1) / 2;
             }
         }
     }
 }
 
 // ---------------------------------------------------------- FP64 tile GEMM
-constexpr int GB_M = 128, GB_N = 128, GB_K = 16, GB_STAGES = 3, GB_THREADS = 256;
-constexpr int GB_SMEM = GB_STAGES * GB_K * (GB_M + GB_N) * 8;
+constexpr int GB_M = 64, GB_N = 128, GB_K = 16, GB_STAGES = 3, GB_THREADS = 128;
+constexpr int GB_PA = GB_M + 4, GB_PB = GB_N + 4;  // row pitches: 32 bytes beyond a bank cycle
+constexpr int GB_SMEM = GB_STAGES * GB_K * (GB_PA + GB_PB) * 8;
+constexpr int GB_PER_SM = 2;
 
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem, int src_bytes)
 {
@@ -193,159 +218,210 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
-// partial[split][a][c] over the edge chunks [chunk0, chunk1) of split
-// `blockIdx.z`: A = psi [n_edges][ldn] (rows beyond n_edges read as zero),
-// B = W [rows][ldc].  Thread (ty, tx) owns rows a0 + 2 ty + 32 i + {0,1} and
-// columns c0 + 2 tx + 32 j + {0,1} (i, j < 4): conflict-free 16-byte
-// shared-memory reads (A broadcast within a warp, B contiguous).
-__global__ void __launch_bounds__(GB_THREADS, 1) psf_wedge_gemm(long long n_edges, int ldn, long long ldc,
-                                                               long long chunks_per_split, long long n_chunks,
-                                                               const double *__restrict__ psi,
-                                                               const double *__restrict__ W,
-                                                               double *__restrict__ partial)
+__device__ __forceinline__ void mma_f64(double (&c)[4], const double (&a)[4], const double (&b)[2])
+{
+    asm volatile("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+                 "{%0,%1,%2,%3};\n"
+                 : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+                 : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
+}
+
+// partial[split][a][c] over the edge chunks of split `blockIdx.z`: A = psi
+// [n_edges][ldn] (rows beyond n_edges read as zero), B = W [rows][ldc].  A
+// warp owns 64 rows x 32 columns as 4 x 4 tiles of 16 x 8.  Rows and columns
+// of a tile are assigned so that a lane's fragments are neighbours in shared
+// memory: fragment row g (g + 8) is row 2g (2g + 1) of the 16, and column n of
+// an even (odd) tile is column 2n (2n + 1) of a pair's 16; every fragment load
+// is then 16 bytes and free of bank conflicts.
+//
+// Bound by the FP64 units: mma.sync m16n8k8 runs at 37.1 TFLOP/s on registers
+// alone, an 8 x 8 outer product of FMAs (the form this replaces) at 31.0.
+// Half of the columns are left out by antisymmetry, 64-row tiles follow N more
+// closely than 128-row ones (ldn is the padded size), and two blocks per SM
+// cover each other's barriers.  16^3 box, N = 128 (11,280 edges): 0.77 ms in
+// two batches against 2.69 ms; the whole tensor 0.96 against 2.97 ms, 20^3,
+// N = 256: 12.9 against 37.2 ms, 11 x 17 x 13, N = 25: 0.06 against 0.36 ms.
+__global__ void __launch_bounds__(GB_THREADS, GB_PER_SM) psf_wedge_gemm(long long n_edges, int ldn, long long ldc,
+                                                                        long long chunks_per_split,
+                                                                        long long n_chunks,
+                                                                        const double *__restrict__ psi,
+                                                                        const double *__restrict__ W,
+                                                                        double *__restrict__ partial)
 {
     extern __shared__ __align__(16) double gsm[];
-    double *As = gsm;                            // [STAGES][K][M]
-    double *Bs = gsm + GB_STAGES * GB_K * GB_M;  // [STAGES][K][N]
-    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+    double *As = gsm;                             // [STAGES][K][PA]
+    double *Bs = gsm + GB_STAGES * GB_K * GB_PA;  // [STAGES][K][PB]
+    const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int wn = (tid >> 5) * 32;
     const int a0 = blockIdx.y * GB_M;
     const long long c0 = (long long)blockIdx.x * GB_N;
     const long long ch0 = (long long)blockIdx.z * chunks_per_split;
     const long long ch1 = min(n_chunks, ch0 + chunks_per_split);
-    const long long nk = max(0ll, ch1 - ch0);
+    const int nk = (int)max(0ll, ch1 - ch0);
 
-    auto load_stage = [&](long long kt, int slot) {
+    auto load_stage = [&](int kt, int slot) {
         const long long e0 = (ch0 + kt) * GB_K;
+        double *sa = As + slot * GB_K * GB_PA, *sb = Bs + slot * GB_K * GB_PB;
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const int q = tid + GB_THREADS * r;  // 1024 16-byte pieces per operand tile
-            const int row = q >> 6, piece = q & 63;
-            const long long e = e0 + row;
-            const bool ok = e < n_edges;
-            const double *srcA = ok ? psi + (size_t)e * ldn + a0 + 2 * piece : psi;
-            cp_async16(As + ((size_t)slot * GB_K + row) * GB_M + 2 * piece, srcA, ok ? 16 : 0);
-            const double *srcB = W + (size_t)e * ldc + c0 + 2 * piece;
-            cp_async16(Bs + ((size_t)slot * GB_K + row) * GB_N + 2 * piece, srcB, 16);
+        for (int r = 0; r < GB_K * GB_M / 2 / GB_THREADS; ++r) {
+            const int q = tid + GB_THREADS * r, row = q / (GB_M / 2), piece = q % (GB_M / 2);
+            const bool ok = e0 + row < n_edges;
+            cp_async16(sa + row * GB_PA + 2 * piece, ok ? psi + (size_t)(e0 + row) * ldn + a0 + 2 * piece : psi,
+                       ok ? 16 : 0);
+        }
+#pragma unroll
+        for (int r = 0; r < GB_K * GB_N / 2 / GB_THREADS; ++r) {
+            const int q = tid + GB_THREADS * r, row = q / (GB_N / 2), piece = q % (GB_N / 2);
+            cp_async16(sb + row * GB_PB + 2 * piece, W + (size_t)(e0 + row) * ldc + c0 + 2 * piece, 16);
         }
     };
 
-    double acc[8][8];
+    double acc[4][4][4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0.0;
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) acc[i][j][q] = 0.0;
 
 #pragma unroll
     for (int s = 0; s < GB_STAGES - 1; ++s) {
         if (s < nk) load_stage(s, s);
         cp_async_commit();
     }
-    for (long long kt = 0; kt < nk; ++kt) {
+    int slot = 0;
+    for (int kt = 0; kt < nk; ++kt) {
         cp_async_wait<GB_STAGES - 2>();
         __syncthreads();
-        const long long nxt = kt + GB_STAGES - 1;
-        if (nxt < nk) load_stage(nxt, (int)(nxt % GB_STAGES));
+        const int nxt = kt + GB_STAGES - 1;
+        if (nxt < nk) load_stage(nxt, slot == 0 ? GB_STAGES - 1 : slot - 1);
         cp_async_commit();
-        const int slot = (int)(kt % GB_STAGES);
-        const double *A = As + (size_t)slot * GB_K * GB_M;
-        const double *B = Bs + (size_t)slot * GB_K * GB_N;
+        const double *A = As + slot * GB_K * GB_PA + 2 * g;
+        const double *B = Bs + slot * GB_K * GB_PB + wn + 2 * g;
+        slot = slot + 1 == GB_STAGES ? 0 : slot + 1;
 #pragma unroll
-        for (int kk = 0; kk < GB_K; ++kk) {
-            double a[8], b[8];
+        for (int k8 = 0; k8 < GB_K; k8 += 8) {
+            double a[4][4], b[4][2];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const double2 v = *reinterpret_cast<const double2 *>(A + kk * GB_M + 2 * ty + 32 * i);
-                a[2 * i] = v.x;
-                a[2 * i + 1] = v.y;
-                const double2 u = *reinterpret_cast<const double2 *>(B + kk * GB_N + 2 * tx + 32 * i);
-                b[2 * i] = u.x;
-                b[2 * i + 1] = u.y;
+            for (int h = 0; h < 2; ++h) {
+                const int k = k8 + 4 * h + t;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const double2 v = *reinterpret_cast<const double2 *>(A + k * GB_PA + 16 * i);
+                    a[i][2 * h] = v.x;
+                    a[i][2 * h + 1] = v.y;
+                }
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const double2 v = *reinterpret_cast<const double2 *>(B + k * GB_PB + 16 * j);
+                    b[2 * j][h] = v.x;
+                    b[2 * j + 1][h] = v.y;
+                }
             }
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
+            for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int j = 0; j < 8; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+                for (int j = 0; j < 4; ++j) mma_f64(acc[i][j], a[i], b[j]);
         }
     }
     cp_async_wait<0>();
 
-    double *P = partial + (size_t)blockIdx.z * ldn * ldc;
+    double *P = partial + ((size_t)blockIdx.z * gridDim.y * GB_M + a0) * ldc + c0 + wn + 4 * t;
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int ii = 0; ii < 2; ++ii) {
-            const int a = a0 + 2 * ty + 32 * i + ii;
+        for (int r = 0; r < 2; ++r) {
+            double *row = P + (size_t)(16 * i + 2 * g + r) * ldc;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const long long c = c0 + 2 * tx + 32 * j;
-                *reinterpret_cast<double2 *>(P + (size_t)a * ldc + c) =
-                    make_double2(acc[2 * i + ii][2 * j], acc[2 * i + ii][2 * j + 1]);
+            for (int j = 0; j < 2; ++j) {
+                const double *even = acc[i][2 * j] + 2 * r, *odd = acc[i][2 * j + 1] + 2 * r;
+                *reinterpret_cast<double2 *>(row + 16 * j) = make_double2(even[0], odd[0]);
+                *reinterpret_cast<double2 *>(row + 16 * j + 2) = make_double2(even[1], odd[1]);
             }
         }
 }
 
-__global__ void psf_wedge_reduce(int N, int ldn, long long ldc, int k0, int kb, int splits,
-                                 const double *__restrict__ partial, const double *__restrict__ lam,
-                                 double *__restrict__ C)
+// A warp sums one row a of one mode k at a time, lanes along j.
+__global__ void __launch_bounds__(256) psf_wedge_reduce(int N, int rows, long long ldc, int k0, int kb, int splits,
+                                                        const double *__restrict__ partial,
+                                                        const double *__restrict__ lam, double *__restrict__ C)
 {
-    const long long total = (long long)kb * N * N;
-    const size_t split_stride = (size_t)ldn * ldc;
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
-         t += (long long)gridDim.x * blockDim.x) {
-        const int j = (int)(t % N);
-        const int a = (int)((t / N) % N);
-        const int kk = (int)(t / ((long long)N * N));
-        const size_t src = (size_t)a * ldc + (size_t)kk * ldn + j;
-        double s = 0.0;
-        for (int p = 0; p < splits; ++p) s += partial[p * split_stride + src];
-        const int k = k0 + kk;
-        C[((size_t)k * N + a) * N + j] = s / lam[k];
+    const int lane = threadIdx.x & 31;
+    const long long nwarps = (long long)gridDim.x * 8;
+    const size_t split_stride = (size_t)rows * ldc;
+    for (long long t = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); t < (long long)kb * N; t += nwarps) {
+        const int kk = (int)(t / N), a = (int)(t % N), k = k0 + kk;
+        const double *src = partial + (size_t)a * ldc + columns_before(N, k0, k) - first_of(k);
+        const double lk = lam[k];
+        double *row = C + ((size_t)k * N + a) * N;
+        if (lane == 0) row[k] = 0.0;
+        for (int j = k + 1 + lane; j < N; j += 32) {
+            double s = 0.0;
+            for (int p = 0; p < splits; ++p) s += __ldcs(src + p * split_stride + j);
+            row[j] = s / lk;
+            C[((size_t)j * N + a) * N + k] = -s / lam[j];
+        }
     }
 }
 
-// Work split of one W batch: GEMM tiles per batch and the number of edge
-// splits that gives the grid about two tiles per SM.
+// Work split of one W batch.  The grid is (column tiles, row tiles, edge
+// splits); the splits are chosen so that the last of its waves over
+// GB_PER_SM blocks per SM is well filled, against the cost of more partial
+// sums: a chunk of a full wave takes about 2.4 us, a block's start and end
+// about eight chunks, a partial sum is written and read once at about 5 TB/s.
 struct WedgePlan {
-    long long n_chunks, rows, ldc, tiles, splits, chunks_per_split;
+    long long n_chunks, rows, ldc, row_tiles, col_tiles, splits, chunks_per_split;
     size_t w_bytes, partial_bytes;
 };
 
-WedgePlan plan_of(const psf_wedge_desc *d, int kb)
+WedgePlan plan_of(const psf_wedge_desc *d, int k0, int kb)
 {
     WedgePlan p{};
     p.n_chunks = (d->n_edges + GB_K - 1) / GB_K;
     p.rows = p.n_chunks * GB_K;
-    p.ldc = (long long)kb * d->ldn;
-    p.tiles = (long long)(d->ldn / GB_M) * (p.ldc / GB_N);
-    const long long want = std::max(1ll, (2ll * 148 + p.tiles - 1) / p.tiles);
-    p.splits = std::max(1ll, std::min({want, 64ll, std::max(1ll, p.n_chunks)}));
-    p.chunks_per_split = std::max(1ll, (p.n_chunks + p.splits - 1) / p.splits);
-    p.splits = std::max(1ll, (p.n_chunks + p.chunks_per_split - 1) / p.chunks_per_split);
+    p.col_tiles = std::max(1ll, (columns_before(d->n_modes, k0, k0 + kb) + GB_N - 1) / GB_N);
+    p.ldc = p.col_tiles * GB_N;
+    p.row_tiles = (d->n_modes + GB_M - 1) / GB_M;
+    const long long tiles = p.row_tiles * p.col_tiles, slots = 148ll * GB_PER_SM;
+    double best = 1e300;
+    p.splits = p.chunks_per_split = 1;
+    for (long long s = 1; s <= std::min(64ll, std::max(1ll, p.n_chunks)); ++s) {
+        const long long per = std::max(1ll, (p.n_chunks + s - 1) / s);
+        const long long used = std::max(1ll, (p.n_chunks + per - 1) / per);
+        const double cost = (double)((tiles * used + slots - 1) / slots) * (double)(per + 8) * 2.4 +
+                            (double)used * (double)(tiles * GB_M * GB_N * 16) / 5e6;
+        if (cost < best) {
+            best = cost;
+            p.splits = used;
+            p.chunks_per_split = per;
+        }
+    }
     p.w_bytes = (size_t)p.rows * p.ldc * sizeof(double);
-    p.partial_bytes = (size_t)p.splits * d->ldn * p.ldc * sizeof(double);
+    p.partial_bytes = (size_t)p.splits * p.row_tiles * GB_M * p.ldc * sizeof(double);
     return p;
 }
 
-// Workspace layout: W of a full batch at offset 0, then the partial sums,
-// sized for the larger of the full batch and the last (shorter) one, whose
-// edge split may differ.
+// Workspace layout: W of the largest batch (the first) at offset 0, then the
+// partial sums, sized for the batch that needs most.
 struct Workspace {
     size_t w_bytes, partial_bytes;
 };
 
 Workspace workspace_of(const psf_wedge_desc *d, int kb)
 {
-    const WedgePlan full = plan_of(d, kb);
-    size_t partial = full.partial_bytes;
-    const int last = d->n_modes % kb;
-    if (last) partial = std::max(partial, plan_of(d, last).partial_bytes);
-    return Workspace{full.w_bytes, partial};
+    Workspace ws{0, 0};
+    for (int k0 = 0; k0 < d->n_modes; k0 += kb) {
+        const WedgePlan q = plan_of(d, k0, std::min(kb, d->n_modes - k0));
+        ws.w_bytes = std::max(ws.w_bytes, q.w_bytes);
+        ws.partial_bytes = std::max(ws.partial_bytes, q.partial_bytes);
+    }
+    return ws;
 }
 
 int check_desc(const psf_wedge_desc *d, int kb)
 {
     if (!d) return fail(PSF_ERR_INVALID, "null wedge descriptor");
-    if (d->n_edges < 0 || d->n_modes < 1 || d->ldn < d->n_modes || d->ldn % GB_M != 0)
+    if (d->n_edges < 0 || d->n_modes < 1 || d->ldn < d->n_modes || d->ldn % 128 != 0)
         return fail(PSF_ERR_INVALID, "wedge descriptor: n_modes >= 1 and ldn a multiple of 128 >= n_modes");
     if (kb < 1 || kb > d->n_modes || kb > WEDGE_KB_MAX)
         return fail(PSF_ERR_INVALID, "k_batch must be in [1, min(n_modes, 64)]");
@@ -419,22 +495,21 @@ extern "C" int psf_pre_advection_tensor(const psf_wedge_desc *d, int32_t k_batch
     const int N = d->n_modes;
     for (int k0 = 0; k0 < N; k0 += k_batch) {
         const int kb = std::min(k_batch, N - k0);
-        const WedgePlan q = plan_of(d, kb);
+        const WedgePlan q = plan_of(d, k0, kb);
         const long long wblocks = std::max(1ll, std::min<long long>((q.rows + 7) / 8, 148ll * 16));
-        psf_wedge_w<<<(unsigned)wblocks, 256, 0, st>>>(d->n_edges, q.rows, d->ldn, k0, kb, d->edge_faces, d->edge_S,
-                                                       d->phi, d->phi_zero_row, W);
+        psf_wedge_w<<<(unsigned)wblocks, 256, 0, st>>>(d->n_edges, q.rows, N, d->ldn, q.ldc, k0, kb, d->edge_faces,
+                                                       d->edge_S, d->phi, d->phi_zero_row, W);
         if (q.n_chunks > 0) {
-            const dim3 grid((unsigned)(q.ldc / GB_N), (unsigned)(d->ldn / GB_M), (unsigned)q.splits);
+            const dim3 grid((unsigned)q.col_tiles, (unsigned)q.row_tiles, (unsigned)q.splits);
             psf_wedge_gemm<<<grid, GB_THREADS, GB_SMEM, st>>>(d->n_edges, d->ldn, q.ldc, q.chunks_per_split,
                                                              q.n_chunks, d->psi, W, partial);
         } else {
             e = cudaMemsetAsync(partial, 0, q.partial_bytes, st);
             if (e != cudaSuccess) return cuda_fail(e, "clearing the partial sums");
         }
-        const long long total = (long long)kb * N * N;
-        const long long rblocks = std::min<long long>((total + 255) / 256, 148ll * 32);
-        psf_wedge_reduce<<<(unsigned)rblocks, 256, 0, st>>>(N, d->ldn, q.ldc, k0, kb, (int)q.splits, partial,
-                                                           d->eigenvalues, C);
+        const long long rblocks = std::min<long long>(((long long)kb * N + 7) / 8, 148ll * 8);
+        psf_wedge_reduce<<<(unsigned)rblocks, 256, 0, st>>>(N, (int)(q.row_tiles * GB_M), q.ldc, k0, kb, (int)q.splits,
+                                                           partial, d->eigenvalues, C);
         e = cudaGetLastError();
         if (e != cudaSuccess) return cuda_fail(e, "advection tensor launch");
     }

@@ -286,7 +286,8 @@ def advection_tensor(dom: Domain, phi_I: np.ndarray, lam: np.ndarray, device=0, 
 
     ``stats``, when given, receives the device time of the tensor kernels
     (``kernel_ms``), the edges with wedge terms, the mode batch and the GEMM's
-    FP64 operation count (``gemm_flops`` = 2 N^2 ldn E over all batches).
+    FP64 operation count (``gemm_flops`` = N^2 (N - 1) E over all batches: the
+    columns j > k of every mode k).
     """
     import torch
 
@@ -323,7 +324,7 @@ def advection_tensor(dom: Domain, phi_I: np.ndarray, lam: np.ndarray, device=0, 
     torch.cuda.synchronize(dev)
     if stats is not None:
         stats.update(kernel_ms=e0.elapsed_time(e1), edges=E, k_batch=kb, ldn=ldn,
-                     gemm_flops=2.0 * N * (N * ldn) * ((E + 15) // 16 * 16))
+                     gemm_flops=1.0 * N * N * (N - 1) * E)
     del ws
     return C if return_device else C.cpu().numpy()
 
