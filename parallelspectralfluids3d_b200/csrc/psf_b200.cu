@@ -295,6 +295,7 @@ __global__ void __launch_bounds__(256) psf_reconstruct(const float *__restrict__
 // (or an earlier, synchronised profiling step).
 constexpr int TRACE_THREADS = 256;
 
+template <class Box>
 __global__ void __launch_bounds__(TRACE_THREADS, 3) psf_trace(float4 *__restrict__ parts, long long P,
                                                  const int32_t *__restrict__ perm,
                                                  const float2 *__restrict__ pairs, GridDev g, TraceParams tp,
@@ -308,7 +309,7 @@ __global__ void __launch_bounds__(TRACE_THREADS, 3) psf_trace(float4 *__restrict
     const uint64_t step = *step_ctr - 1ull;
     for (bool first = true; i < P; i += stride, first = false) {
         if (!first) p = parts[i];
-        parts[i] = advance_particle(p, g, pairs, tp, step, perm, (size_t)i);
+        parts[i] = advance_particle<Box>(p, g, pairs, tp, step, perm, (size_t)i);
     }
 }
 
@@ -437,7 +438,7 @@ int launch_reconstruct(const PlainDev &d, cudaStream_t st, bool after_kernel)
 int trace_blocks_per_sm()
 {
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, psf_trace, TRACE_THREADS, 0) != cudaSuccess ||
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, psf_trace<CentredBox>, TRACE_THREADS, 0) != cudaSuccess ||
         per_sm < 1)
         per_sm = 4;
     return per_sm;
@@ -450,7 +451,7 @@ int launch_trace(const PlainDev &d, cudaStream_t st, bool after_kernel)
         std::min<long long>((d.P + TRACE_THREADS - 1) / TRACE_THREADS, std::max(1, d.trace_blocks));
     PdlLaunch L((unsigned)blocks, TRACE_THREADS, st);
     if (!after_kernel) L.cfg.numAttrs = 0;
-    cudaError_t e = cudaLaunchKernelEx(&L.cfg, psf_trace, d.parts, (long long)d.P, (const int32_t *)d.perm,
+    cudaError_t e = cudaLaunchKernelEx(&L.cfg, d.grid.centered ? psf_trace<CentredBox> : psf_trace<AnyBox>, d.parts, (long long)d.P, (const int32_t *)d.perm,
                                        d.trace_pairs, d.grid, d.tp, d.trace_ctr);
     return e == cudaSuccess ? PSF_OK : cuda_fail(e, "psf_trace launch");
 }

@@ -560,6 +560,7 @@ __global__ void psf_batch_pack(const GroupDev *__restrict__ groups, const SlotDe
 // sums of the slots' particle counts; a particle finds its slot by binary
 // search in shared memory.  Slots that did not advance this step (step limit
 // reached) are skipped.
+template <bool ALL_CENTRED>
 __global__ void __launch_bounds__(128, 5) psf_batch_trace(const GroupDev *__restrict__ groups,
                                                           const SlotDev *__restrict__ slots,
                                                           const long long *__restrict__ prefix, int n_slots)
@@ -610,7 +611,10 @@ __global__ void __launch_bounds__(128, 5) psf_batch_trace(const GroupDev *__rest
         if (!live) continue;
         const size_t idx = base + (size_t)gi;
         float4 p = G->parts[idx];
-        p = advance_particle(p, G->grid, pairs, tp, step, G->perm, idx);
+        if (ALL_CENTRED || G->grid.centered)
+            p = advance_particle<CentredBox>(p, G->grid, pairs, tp, step, G->perm, idx);
+        else
+            p = advance_particle<AnyBox>(p, G->grid, pairs, tp, step, G->perm, idx);
         G->parts[idx] = p;
     }
 }
@@ -730,16 +734,19 @@ int launch_batch_pack(const GroupDev *groups, const SlotDev *slots, int slot_glo
 int batch_trace_grid(int num_sms)
 {
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, psf_batch_trace, 128, 0) != cudaSuccess || per_sm < 1)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, psf_batch_trace<true>, 128, 0) != cudaSuccess || per_sm < 1)
         per_sm = 4;
     return num_sms * per_sm;
 }
 
 int launch_batch_trace(const GroupDev *groups, const SlotDev *slots, const long long *prefix, int n_slots, int grid,
-                       cudaStream_t st)
+                       bool all_centred, cudaStream_t st)
 {
     if (n_slots < 1 || n_slots > BATCH_MAX_ALL_SLOTS) return fail(PSF_ERR_INVALID, "slot count out of range");
-    psf_batch_trace<<<grid, 128, 0, st>>>(groups, slots, prefix, n_slots);
+    if (all_centred)
+        psf_batch_trace<true><<<grid, 128, 0, st>>>(groups, slots, prefix, n_slots);
+    else
+        psf_batch_trace<false><<<grid, 128, 0, st>>>(groups, slots, prefix, n_slots);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? PSF_OK : cuda_fail(e, "psf_batch_trace launch");
 }

@@ -143,6 +143,7 @@ struct psf_batch {
     int ksplit = 1;   // K ranges per contraction row tile
     int gemm_ctas = 148;
     int trace_ctas = 592;
+    bool all_centred = true;  // every basis has a centred box (GridDev::centered)
     double tuned_ms = 0.0;
     psf::OrderBufs order{};
     int64_t pmax_all = 0;
@@ -339,6 +340,7 @@ int upload_tables(psf_batch *B)
         const HostGroup &G = B->groups[gi];
         psf::GroupDev &d = gd[gi];
         d.grid = psf::make_grid_dev(G.grid);
+        if (!d.grid.centered) B->all_centred = false;
         d.N = G.N;
         d.Nj = G.Nj;
         d.cap = G.cap;
@@ -494,7 +496,8 @@ int autotune(psf_batch *B, int need_bn)
 int launch_step(psf_batch *B, cudaStream_t st)
 {
     PSF_CHECK(launch_tc_part(B, st, B->use_fused));
-    PSF_CHECK(psf::launch_batch_trace(B->d_groups, B->d_slots, B->d_prefix, B->n_slots(), B->trace_ctas, st));
+    PSF_CHECK(psf::launch_batch_trace(B->d_groups, B->d_slots, B->d_prefix, B->n_slots(), B->trace_ctas,
+                                      B->all_centred, st));
     return PSF_OK;
 }
 
@@ -1004,7 +1007,8 @@ static int profile(psf_batch *B, double *kernel_ms, int32_t n, bool fused)
         cudaEventRecord(ev[3], st);
     }
     if (rc == PSF_OK)
-        rc = psf::launch_batch_trace(B->d_groups, B->d_slots, B->d_prefix, B->n_slots(), B->trace_ctas, st);
+        rc = psf::launch_batch_trace(B->d_groups, B->d_slots, B->d_prefix, B->n_slots(), B->trace_ctas,
+                                      B->all_centred, st);
     cudaEventRecord(ev[nk], st);
     cudaError_t e = cudaStreamSynchronize(st);
     if (rc == PSF_OK && e != cudaSuccess) rc = psf::cuda_fail(e, "profiled step");

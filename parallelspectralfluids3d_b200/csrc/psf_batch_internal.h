@@ -112,7 +112,7 @@ int max_fused_grid(int bn_max, int num_sms);
 int launch_batch_state(const GroupDev *groups, SlotDev *slots, int n_slots, cudaStream_t st);
 // prefix[s] = particles of slots 0..s-1 (occupied slots only); n_slots + 1 entries.
 int launch_batch_trace(const GroupDev *groups, const SlotDev *slots, const long long *prefix, int n_slots, int grid,
-                       cudaStream_t st);
+                       bool all_centred, cudaStream_t st);
 int launch_batch_pack(const GroupDev *groups, const SlotDev *slots, int slot_global, cudaStream_t st);
 int batch_trace_grid(int num_sms);
 

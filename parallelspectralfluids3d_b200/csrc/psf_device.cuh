@@ -171,35 +171,133 @@ __device__ __forceinline__ float3 interpolate(const CellCache &c, const float3 &
     return v;
 }
 
-// Velocity at a position; `c` carries the last gathered cell, and the
-// samples are loaded again only when the position lies in another cell.
-// When the box is centred (shift == -mn exactly, as for every domain built
-// here) the reference's index coordinate (shift + p) / h and the weight
-// coordinate (p - mn) / h are the same float, so it is computed once.
-__device__ __forceinline__ float3 velocity_cached(const GridDev &g, const float2 *__restrict__ pairs, float px,
-                                                  float py, float pz, CellCache &c, bool &have)
-{
-    float3 gw;
-    gw.x = (px - g.mn[0]) * g.inv_h;
-    gw.y = (py - g.mn[1]) * g.inv_h;
-    gw.z = (pz - g.mn[2]) * g.inv_h;
-    int kx, ky, kz;
-    if (g.centered) {
-        kx = clampi(__float2int_rd(2.0f * gw.x), -1, 2 * g.nx);
-        ky = clampi(__float2int_rd(2.0f * gw.y), -1, 2 * g.ny);
-        kz = clampi(__float2int_rd(2.0f * gw.z), -1, 2 * g.nz);
-    } else {
+// Velocity at a position of a box whose index and weight coordinates differ;
+// `c` carries the last gathered cell, and the samples are loaded again only
+// when the position lies in another cell.
+struct AnyBox {
+    CellCache c;
+    bool have = false;
+    __device__ __forceinline__ float3 velocity(const GridDev &g, const float2 *__restrict__ pairs, float px, float py,
+                                               float pz)
+    {
+        int kx, ky, kz;
         cell_key(g, px, py, pz, kx, ky, kz);
+        if (!have || kx != c.kx || ky != c.ky || kz != c.kz) {
+            c.kx = kx;
+            c.ky = ky;
+            c.kz = kz;
+            gather_cell(g, pairs, kx, ky, kz, c);
+            have = true;
+        }
+        return interpolate(c, make_float3((px - g.mn[0]) * g.inv_h, (py - g.mn[1]) * g.inv_h,
+                                          (pz - g.mn[2]) * g.inv_h));
     }
-    if (!have || kx != c.kx || ky != c.ky || kz != c.kz) {
-        c.kx = kx;
-        c.ky = ky;
-        c.kz = kz;
-        gather_cell(g, pairs, kx, ky, kz, c);
-        have = true;
+};
+
+// One staggered component in a half-cell: its value and its y, x and xy
+// differences on the two z planes of its stencil.
+struct Trilinear {
+    float v0, dy0, dx0, dxy0, v1, dy1, dx1, dxy1;
+    __device__ __forceinline__ float at(float tx, float ty, float tz) const
+    {
+        const float a = fmaf(tx, fmaf(ty, dxy0, dx0), fmaf(ty, dy0, v0));
+        const float b = fmaf(tx, fmaf(ty, dxy1, dx1), fmaf(ty, dy1, v1));
+        return mixf(a, b, tz);
     }
-    return interpolate(c, gw);
-}
+};
+
+// The same on a centred box (shift == -mn exactly, as for every domain built
+// here), where the reference's index coordinate (shift + p) / h and the weight
+// coordinate (p - mn) / h are the same number.  A half-cell is k = floor(2 gw)
+// per axis; in it the coordinate from the whole-cell origin (own axis of a
+// component) and the one from the half-shifted origin (other axes) differ by
+// 1/2 either way, and the smaller of them is the place in the half-cell.  So
+// a position lies in the gathered half-cell when that minimum is in [0, 1/2]
+// (an unsigned compare of the bits; the interpolant is continuous, so either
+// side may take a shared boundary), and the two coordinates are all the
+// interpolation needs.  In the lowest half-cell the half-shifted stencil has
+// one sample on both sides, so its coordinate does not matter there and keeps
+// the unclamped origin.
+//
+// Bound by the latency and L1 lookups of the gathers (RK1, which has one per
+// particle and little else, takes 80 us where RK4 takes 102).  Against three
+// cell keys and nested lerps, 16 x 262,144 particles on the 32^3 box with a
+// sphere, RK4: 102 against 111 us at 0.001 voxel per step, 129 against 133 us
+// at 0.03; 513 x 16,384 on three domains: 284 against 297 us.  Storing the
+// pairs in bricks of 4 x 2 x 2 voxels made RK1 73 us but RK4 139 us (the
+// places cost more in the repeated gathers) and the 512-slot reconstruction
+// 353 against 302 us; storing every face once (24 loads of 4 bytes) was slower
+// at every density.
+struct CentredBox {
+    float ox, oy, oz;     // whole-cell origin
+    float sx, sy, sz;     // half-shifted origin
+    Trilinear x, y, z;
+    bool have = false;
+
+    __device__ __forceinline__ void gather(const GridDev &g, const float2 *__restrict__ pairs, float qx, float qy,
+                                           float qz)
+    {
+        const int kx = clampi(__float2int_rd(2.0f * (qx * g.inv_h)), 0, 2 * g.nx - 1);
+        const int ky = clampi(__float2int_rd(2.0f * (qy * g.inv_h)), 0, 2 * g.ny - 1);
+        const int kz = clampi(__float2int_rd(2.0f * (qz * g.inv_h)), 0, 2 * g.nz - 1);
+        const int xO = kx >> 1, yO = ky >> 1, zO = kz >> 1;
+        const int xr = (kx - 1) >> 1, yr = (ky - 1) >> 1, zr = (kz - 1) >> 1;
+        ox = (float)xO;
+        oy = (float)yO;
+        oz = (float)zO;
+        sx = (float)xr + 0.5f;
+        sy = (float)yr + 0.5f;
+        sz = (float)zr + 0.5f;
+        const int xM = max(xr, 0), xP = min(xr + 1, g.nx - 1);
+        const uint32_t nx = (uint32_t)g.nx, nxy = (uint32_t)(g.nx * g.ny), V = nxy * (uint32_t)g.nz;
+        const uint32_t yM = (uint32_t)max(yr, 0) * nx, yP = (uint32_t)min(yr + 1, g.ny - 1) * nx;
+        const uint32_t zM = (uint32_t)max(zr, 0) * nxy, zP = (uint32_t)min(zr + 1, g.nz - 1) * nxy;
+        const uint32_t yW = (uint32_t)yO * nx, zW = (uint32_t)zO * nxy;
+        const float2 *__restrict__ py = pairs + V;
+        const float2 *__restrict__ pz = pairs + 2 * (size_t)V;
+        const float2 x00 = __ldg(pairs + (zM + yM + xO)), x10 = __ldg(pairs + (zM + yP + xO));
+        const float2 x01 = __ldg(pairs + (zP + yM + xO)), x11 = __ldg(pairs + (zP + yP + xO));
+        const float2 y00 = __ldg(py + (zM + yW + xM)), y10 = __ldg(py + (zM + yW + xP));
+        const float2 y01 = __ldg(py + (zP + yW + xM)), y11 = __ldg(py + (zP + yW + xP));
+        const float2 z00 = __ldg(pz + (zW + yM + xM)), z01 = __ldg(pz + (zW + yP + xM));
+        const float2 z10 = __ldg(pz + (zW + yM + xP)), z11 = __ldg(pz + (zW + yP + xP));
+        auto plane = [](float v, float vy, float vx, float vxy, float &o, float &dy, float &dx, float &dxy) {
+            o = v;
+            dy = vy - v;
+            dx = vx - v;
+            dxy = (vxy - vx) - dy;
+        };
+        plane(x00.x, x10.x, x00.y, x10.y, x.v0, x.dy0, x.dx0, x.dxy0);
+        plane(x01.x, x11.x, x01.y, x11.y, x.v1, x.dy1, x.dx1, x.dxy1);
+        plane(y00.x, y00.y, y10.x, y10.y, y.v0, y.dy0, y.dx0, y.dxy0);
+        plane(y01.x, y01.y, y11.x, y11.y, y.v1, y.dy1, y.dx1, y.dxy1);
+        plane(z00.x, z01.x, z10.x, z11.x, z.v0, z.dy0, z.dx0, z.dxy0);
+        plane(z00.y, z01.y, z10.y, z11.y, z.v1, z.dy1, z.dx1, z.dxy1);
+    }
+
+    __device__ __forceinline__ static bool inside(float a, float b)
+    {
+        return __float_as_uint(fminf(a, b)) <= 0x3F000000u;  // [0, 1/2]
+    }
+
+    __device__ __forceinline__ float3 velocity(const GridDev &g, const float2 *__restrict__ pairs, float px, float py,
+                                               float pz)
+    {
+        const float qx = px - g.mn[0], qy = py - g.mn[1], qz = pz - g.mn[2];
+        if (!have) {
+            gather(g, pairs, qx, qy, qz);
+            have = true;
+        } else {
+            const bool same = inside(fmaf(qx, g.inv_h, -ox), fmaf(qx, g.inv_h, -sx)) &&
+                              inside(fmaf(qy, g.inv_h, -oy), fmaf(qy, g.inv_h, -sy)) &&
+                              inside(fmaf(qz, g.inv_h, -oz), fmaf(qz, g.inv_h, -sz));
+            if (!same) gather(g, pairs, qx, qy, qz);
+        }
+        const float ax = fmaf(qx, g.inv_h, -ox), ay = fmaf(qy, g.inv_h, -oy), az = fmaf(qz, g.inv_h, -oz);
+        const float bx = fmaf(qx, g.inv_h, -sx), by = fmaf(qy, g.inv_h, -sy), bz = fmaf(qz, g.inv_h, -sz);
+        return make_float3(x.at(ax, by, bz), y.at(bx, ay, bz), z.at(bx, by, az));
+    }
+};
 
 __device__ __forceinline__ float clampf(float v, float lo, float hi) { return fminf(fmaxf(v, lo), hi); }
 
@@ -223,34 +321,34 @@ __device__ __forceinline__ float div6(float x)
 // generator keyed by the caller-order index `perm[idx]` when the lifetime ran
 // out (read only then).  `step` is the index of the step being taken (0 for
 // the first).
+template <class Box>
 __device__ __forceinline__ float4 advance_particle(float4 p, const GridDev &g, const float2 *__restrict__ u,
                                                    const TraceParams &tp, uint64_t step,
                                                    const int32_t *__restrict__ perm, size_t idx)
 {
     if (p.w > 0.f) {
         const float dt = tp.dt;
-        CellCache c;
-        bool have = false;
+        Box box;
         float3 v;
         if (tp.rk4) {
-            const float3 k1 = velocity_cached(g, u, p.x, p.y, p.z, c, have);
+            const float3 k1 = box.velocity(g, u, p.x, p.y, p.z);
             float qx = clampf(p.x + 0.5f * dt * k1.x, g.mn[0], g.mx[0]);
             float qy = clampf(p.y + 0.5f * dt * k1.y, g.mn[1], g.mx[1]);
             float qz = clampf(p.z + 0.5f * dt * k1.z, g.mn[2], g.mx[2]);
-            const float3 k2 = velocity_cached(g, u, qx, qy, qz, c, have);
+            const float3 k2 = box.velocity(g, u, qx, qy, qz);
             qx = clampf(p.x + 0.5f * dt * k2.x, g.mn[0], g.mx[0]);
             qy = clampf(p.y + 0.5f * dt * k2.y, g.mn[1], g.mx[1]);
             qz = clampf(p.z + 0.5f * dt * k2.z, g.mn[2], g.mx[2]);
-            const float3 k3 = velocity_cached(g, u, qx, qy, qz, c, have);
+            const float3 k3 = box.velocity(g, u, qx, qy, qz);
             qx = clampf(p.x + dt * k3.x, g.mn[0], g.mx[0]);
             qy = clampf(p.y + dt * k3.y, g.mn[1], g.mx[1]);
             qz = clampf(p.z + dt * k3.z, g.mn[2], g.mx[2]);
-            const float3 k4 = velocity_cached(g, u, qx, qy, qz, c, have);
+            const float3 k4 = box.velocity(g, u, qx, qy, qz);
             v.x = div6(k1.x + 2.f * k2.x + 2.f * k3.x + k4.x);
             v.y = div6(k1.y + 2.f * k2.y + 2.f * k3.y + k4.y);
             v.z = div6(k1.z + 2.f * k2.z + 2.f * k3.z + k4.z);
         } else {
-            v = velocity_cached(g, u, p.x, p.y, p.z, c, have);
+            v = box.velocity(g, u, p.x, p.y, p.z);
         }
         p.x = clampf(p.x + dt * v.x, g.mn[0], g.mx[0]);
         p.y = clampf(p.y + dt * v.y, g.mn[1], g.mx[1]);
