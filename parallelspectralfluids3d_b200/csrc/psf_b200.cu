@@ -378,34 +378,6 @@ int launch_unorder_particles(const PlainDev &d, const OrderBufs &o, cudaStream_t
 }
 
 // ------------------------------------------------------------- launchers
-int launch_contract_state(const PlainDev &d, cudaStream_t st)
-{
-    const int CH = (d.Np + 127) / 128;
-    const dim3 grid(d.N * d.S), block(256);
-#define PSF_CASE(n)                                                                                   \
-    case n:                                                                                           \
-        psf_contract_state<n><<<grid, block, 0, st>>>(d.C, d.N, d.Np, d.S, d.w, d.w_next, d.dwpart,  \
-                                                      d.lam, d.force, d.sp, d.ticket, d.step_ctr,    \
-                                                      d.step_ctr_next);                              \
-        break;
-    switch (CH) {
-        PSF_CASE(1)
-        PSF_CASE(2)
-        PSF_CASE(3)
-        PSF_CASE(4)
-        PSF_CASE(5)
-        PSF_CASE(6)
-        PSF_CASE(7)
-        PSF_CASE(8)
-    default:
-        return fail(PSF_ERR_UNSUPPORTED, "mode count above the supported maximum");
-    }
-#undef PSF_CASE
-    cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? PSF_OK : cuda_fail(e, "psf_contract_state launch");
-}
-
-
 // Launch configuration of a step kernel that may start while the previous
 // kernel in the stream finishes (programmatic stream serialisation).
 struct PdlLaunch {
@@ -423,6 +395,34 @@ struct PdlLaunch {
         cfg.numAttrs = 1;
     }
 };
+
+int launch_contract_state(const PlainDev &d, cudaStream_t st, bool after_kernel)
+{
+    const int CH = (d.Np + 127) / 128;
+    PdlLaunch L((unsigned)(d.N * d.S), 256, st);
+    if (!after_kernel) L.cfg.numAttrs = 0;
+    cudaError_t e = cudaSuccess;
+#define PSF_CASE(n)                                                                                             \
+    case n:                                                                                                     \
+        e = cudaLaunchKernelEx(&L.cfg, psf_contract_state<n>, d.C, (int)d.N, (int)d.Np, (int)d.S,               \
+                               (const double *)d.w, d.w_next, d.dwpart, d.lam, d.force, d.sp, d.ticket,         \
+                               (const unsigned long long *)d.step_ctr, d.step_ctr_next);                        \
+        break;
+    switch (CH) {
+        PSF_CASE(1)
+        PSF_CASE(2)
+        PSF_CASE(3)
+        PSF_CASE(4)
+        PSF_CASE(5)
+        PSF_CASE(6)
+        PSF_CASE(7)
+        PSF_CASE(8)
+    default:
+        return fail(PSF_ERR_UNSUPPORTED, "mode count above the supported maximum");
+    }
+#undef PSF_CASE
+    return e == cudaSuccess ? PSF_OK : cuda_fail(e, "psf_contract_state launch");
+}
 
 int launch_reconstruct(const PlainDev &d, cudaStream_t st, bool after_kernel)
 {

@@ -105,7 +105,7 @@ extern thread_local std::string g_last_error;
 int fail(int code, const std::string &msg);
 int cuda_fail(cudaError_t e, const char *what);
 
-int launch_contract_state(const PlainDev &d, cudaStream_t st);
+int launch_contract_state(const PlainDev &d, cudaStream_t st, bool after_kernel = false);
 // `after_kernel`: the launch directly follows a kernel in the stream and may
 // start during that kernel's tail (programmatic dependent launch).
 int launch_reconstruct(const PlainDev &d, cudaStream_t st, bool after_kernel = true);
