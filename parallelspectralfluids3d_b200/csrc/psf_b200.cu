@@ -438,7 +438,7 @@ int launch_reconstruct(const PlainDev &d, cudaStream_t st, bool after_kernel)
 int trace_blocks_per_sm()
 {
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, psf_trace<CentredBox>, TRACE_THREADS, 0) != cudaSuccess ||
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, psf_trace<CentredBox<PairField>>, TRACE_THREADS, 0) != cudaSuccess ||
         per_sm < 1)
         per_sm = 4;
     return per_sm;
@@ -451,7 +451,7 @@ int launch_trace(const PlainDev &d, cudaStream_t st, bool after_kernel)
         std::min<long long>((d.P + TRACE_THREADS - 1) / TRACE_THREADS, std::max(1, d.trace_blocks));
     PdlLaunch L((unsigned)blocks, TRACE_THREADS, st);
     if (!after_kernel) L.cfg.numAttrs = 0;
-    cudaError_t e = cudaLaunchKernelEx(&L.cfg, d.grid.centered ? psf_trace<CentredBox> : psf_trace<AnyBox>, d.parts, (long long)d.P, (const int32_t *)d.perm,
+    cudaError_t e = cudaLaunchKernelEx(&L.cfg, d.grid.centered ? psf_trace<CentredBox<PairField>> : psf_trace<AnyBox>, d.parts, (long long)d.P, (const int32_t *)d.perm,
                                        d.trace_pairs, d.grid, d.tp, d.trace_ctr);
     return e == cudaSuccess ? PSF_OK : cuda_fail(e, "psf_trace launch");
 }

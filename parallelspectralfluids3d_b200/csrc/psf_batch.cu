@@ -17,7 +17,7 @@
 // psf_batch_step_tc is one persistent kernel over the tiles of every basis:
 // warp 0 streams 128-row A tiles and the W tile through a TMA ring of
 // shared-memory stages (128-byte swizzle, no multicast), warp 1 issues the
-// tcgen05.mma chain for a tile into one of two TMEM accumulators, warps 2-5
+// tcgen05.mma chain for a tile into one of two TMEM accumulators, warps 2-9
 // drain the other accumulator (tcgen05.ld) and run the epilogue, so loads,
 // MMAs and epilogue overlap.  In the default (fused) step one cooperative
 // launch runs the contraction, the FP64 state update of every slot and the
@@ -114,7 +114,7 @@ __device__ __forceinline__ double warp_allsum(double v)
     return v;
 }
 
-__device__ __forceinline__ void epilogue_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+__device__ __forceinline__ void epilogue_bar() { asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory"); }
 
 // Grid-wide barrier of a cooperative launch: arrive, then wait (bounded) until
 // `target` arrivals were counted.  Called by one thread per CTA after a CTA
@@ -145,14 +145,14 @@ __device__ __forceinline__ void split_bf16(double x, __nv_bfloat16 *hi, __nv_bfl
     *lo = __float2bfloat16_rn((float)(x - (double)__bfloat162float(h)));
 }
 
-// FP64 update of one slot by the 128 epilogue threads of a CTA, in the
+// FP64 update of one slot by the epilogue threads of a CTA, in the
 // reference's order (psfsolver.cpp:37-59), then the new state's FP32 copy and
-// BF16 hi/lo split.  Energy sums: per warp (shuffles), then the 4 warps in
+// BF16 hi/lo split.  Energy sums: per warp (shuffles), then the warps in
 // fixed order, so the result does not depend on timing.
 __device__ void state_update_cta(const GroupDev *__restrict__ groups, SlotDev &s, int et, double *red)
 {
     const int lane = et & 31, ew = et >> 5;
-    if (!s.active) return;  // uniform over the 128 threads
+    if (!s.active) return;  // uniform over the threads
     if (s.target != 0ull && s.step >= s.target) {
         if (et == 0) s.stepped = 0;
         return;
@@ -161,7 +161,7 @@ __device__ void state_update_cta(const GroupDev *__restrict__ groups, SlotDev &s
     const int b = s.slot, N = s.n_modes, parts = G.nparts;
     double *w = G.w + (size_t)b * G.N;
     double e1 = 0.0, e2 = 0.0;
-    for (int i = et; i < N; i += 128) {
+    for (int i = et; i < N; i += EPI_THREADS) {
         double dw = 0.0;
         const double *dp = G.dwpart + (size_t)i * parts * G.cap + b;
         for (int p = 0; p < parts; ++p) dw += dp[(size_t)p * G.cap];
@@ -175,15 +175,19 @@ __device__ void state_update_cta(const GroupDev *__restrict__ groups, SlotDev &s
     e2 = warp_allsum(e2);
     if (lane == 0) {
         red[ew] = e1;
-        red[4 + ew] = e2;
+        red[EPI_WARPS + ew] = e2;
     }
     epilogue_bar();
-    e1 = red[0] + red[1] + red[2] + red[3];
-    e2 = red[4] + red[5] + red[6] + red[7];
+    e1 = e2 = 0.0;
+#pragma unroll
+    for (int i = 0; i < EPI_WARPS; ++i) {
+        e1 += red[i];
+        e2 += red[EPI_WARPS + i];
+    }
     const double scale = (s.flags & PSF_FLAG_RENORM) ? sqrt(e1 / e2) : 1.0;
     __nv_bfloat16 *Whi = reinterpret_cast<__nv_bfloat16 *>(G.W) + (size_t)b * G.Nj;
     __nv_bfloat16 *Wlo = Whi + (size_t)G.bn * G.Nj;
-    for (int i = et; i < N; i += 128) {
+    for (int i = et; i < N; i += EPI_THREADS) {
         double v = w[i] * scale;
         v *= exp(s.visc_signed * G.lam[i] * s.dt);
         if (s.flags & PSF_FLAG_FORCING) v += s.dt * G.force[(size_t)b * G.N + i];
@@ -199,7 +203,8 @@ __device__ void state_update_cta(const GroupDev *__restrict__ groups, SlotDev &s
 }
 
 // One launch of the tensor-core step.  Warp 0: TMA producer; warp 1: MMA
-// issuer; warps 2-5: TMEM epilogue.  Unfused launches run their contraction
+// issuer; warps 2-9: TMEM epilogue, two per lane quarter, which take every other
+// 32 columns.  Unfused launches run their contraction
 // or reconstruction units.  A fused launch (cooperative) is one whole step of
 // the coefficient pipeline: the epilogue warps first update every slot's
 // state from the contraction partials of the previous launch (FP64, one CTA
@@ -224,7 +229,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) psf_batch_step_tc(const __gri
     uint64_t *acc_empty = acc_full + 2;
     uint64_t *wready = acc_empty + 2;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(wready + 1);
-    double *red = reinterpret_cast<double *>(wready + 2);  // 8 doubles (bytes 8*(2*STAGES+6) .. +64)
+    double *red = reinterpret_cast<double *>(wready + 2);  // 2 EPI_WARPS doubles (from byte 8 (2 STAGES + 6))
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int *err = args.err;
@@ -237,7 +242,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) psf_batch_step_tc(const __gri
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&acc_full[b], 1);
-            mbar_init(&acc_empty[b], 128);
+            mbar_init(&acc_empty[b], EPI_THREADS);
         }
         mbar_init(wready, 1);
         mbar_fence_init();
@@ -371,6 +376,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) psf_batch_step_tc(const __gri
     } else {
         // -------------------------------------------------------- epilogue
         const int q = warp & 3;   // TMEM lanes 32q .. 32q+31 belong to this warp
+        const int first = 32 * ((warp - 2) >> 2);  // and columns first + 64 i .. + 32
         const int row = q * 32 + lane;
         int abuf = 0;
         uint32_t aphase = 0;
@@ -397,26 +403,24 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) psf_batch_step_tc(const __gri
             const GemmGroup &G = unit_group<MODE>(args, t, recon, &lt);
             const Unit un = decode_unit(G, lt);
             const int outer = un.outer, inner = un.inner;
-            // Contraction: the state values of this warp's rows for the first
-            // slots are loaded while the accumulator is still being computed.
-            // With at most 64 MMA columns both 32-slot chunks are loaded up
-            // front; with more, each later chunk is loaded one chunk ahead of
-            // its use (two ahead measured 22 % slower at 256 columns).
-            constexpr bool kTwoAhead = BN_MAX <= 64;
-            float wa[32], wb[32];
+            // Two epilogue warps per lane quarter instead of one took the
+            // contraction of 513 slots from 77.6 to 60 us and of 64 slots of
+            // N = 384 from 52 to 45 us: with one, a CTA's last tiles waited
+            // for the epilogue.
+            // Contraction: the state values of this warp's rows for its first
+            // slots are loaded while the accumulator is still being computed,
+            // those of a later chunk one chunk ahead of its use.
+            float wa[32];
             const int a_row = inner * 128 + row;
             const bool arow = !recon && a_row < G.n_rows;
-            auto load_w = [&](float(&dst)[32], int c0) {
+            auto load_w = [&](int c0) {
 #pragma unroll
                 for (int c = 0; c < 32; ++c) {
                     const int b = c0 + c;
-                    dst[c] = (arow && b < G.cap) ? G.wf[(size_t)b * G.ldw + a_row] : 0.f;
+                    wa[c] = (arow && b < G.cap) ? G.wf[(size_t)b * G.ldw + a_row] : 0.f;
                 }
             };
-            if (!recon) {
-                load_w(wa, 0);
-                if (kTwoAhead && 32 < G.bn) load_w(wb, 32);
-            }
+            if (!recon && first < G.bn) load_w(first);
             bool ok = mbar_wait(&acc_full[abuf], aphase, err, ERR_WAIT_ACC_FULL);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
@@ -425,55 +429,52 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) psf_batch_step_tc(const __gri
             if (!recon) {
                 // dw partial of mode k = outer over this warp's 32 rows a:
                 // sum_a w[a][b] Y[a][b] for every slot b, in FP32.
-                auto chunk = [&](int c0, float(&wv)[32]) {
+                for (int c0 = first; c0 < G.bn; c0 += 64) {
                     float y[32];
                     tmem_ld32(tbase + (uint32_t)c0, y);
 #pragma unroll
-                    for (int c = 0; c < 32; ++c) y[c] *= wv[c];
-                    if (kTwoAhead) {
-                        if (c0 + 64 < G.bn) load_w(wv, c0 + 64);
-                    } else if (c0 + 32 < G.bn) {
-                        load_w(wv, c0 + 32);
-                    }
+                    for (int c = 0; c < 32; ++c) y[c] *= wa[c];
+                    if (c0 + 64 < G.bn) load_w(c0 + 64);
                     const float s = warp_reduce_scatter32f(y, lane);
                     const int b = c0 + lane;
                     if (b < G.cap)
                         G.dwpart[((size_t)outer * G.nparts + (inner * G.ksplit + un.ks) * 4 + q) * G.cap + b] =
                             (double)s;
-                };
-                if (kTwoAhead) {
-                    for (int c0 = 0; c0 < G.bn; c0 += 64) {
-                        chunk(c0, wa);
-                        if (c0 + 32 < G.bn) chunk(c0 + 32, wb);
-                    }
-                } else {
-                    for (int c0 = 0; c0 < G.bn; c0 += 32) chunk(c0, wa);
                 }
             } else {
                 // Face velocities of this warp's 32 rows, scattered into the
-                // per-voxel face pairs (each face lands in its two voxels) of
-                // every slot that stepped: the tracer reads no others, so an
-                // empty or finished slot costs no stores.
+                // field of every slot that stepped (a face lands in one place,
+                // or in the pairs of its two voxels): the tracer reads no
+                // others, so an empty or finished slot costs no stores.  The
+                // stores bound this launch once the slots outnumber the modes
+                // (FACE_FIELD_DENSITY has the figures).
                 const long long f = (long long)inner * 128 + row;
                 const bool frow = f < G.n_rows;
-                const int32_t d0 = frow ? __ldg(G.pair_dst + 2 * f) : -1;
-                const int32_t d1 = frow ? __ldg(G.pair_dst + 2 * f + 1) : -1;
-                for (int c0 = 0; c0 < G.bn; c0 += 32) {
+                const int32_t d0 = frow ? __ldg(G.field_dst + 2 * f) : -1;
+                const int32_t d1 = frow ? __ldg(G.field_dst + 2 * f + 1) : -1;
+                const size_t step = (size_t)G.field_floats;
+                const bool twice = __any_sync(0xffffffffu, d1 >= 0);
+                for (int c0 = first; c0 < G.bn; c0 += 64) {
                     const int bl = c0 + lane;
                     const unsigned stepped =
                         __ballot_sync(0xffffffffu, bl < G.cap && G.slot_of[bl].stepped != 0);
                     float y[32];
                     tmem_ld32(tbase + (uint32_t)c0, y);
-                    if (frow && stepped) {
+                    auto put = [&](int32_t place) {
+                        float *p = G.field + (size_t)c0 * step + max(place, 0);
+                        if (stepped == 0xffffffffu) {
 #pragma unroll
-                        for (int c = 0; c < 32; ++c) {
-                            const int b = c0 + c;
-                            if ((stepped >> c) & 1u) {
-                                float *pr = G.pairs + (size_t)b * G.pair_floats;
-                                if (d0 >= 0) pr[d0] = y[c];
-                                if (d1 >= 0) pr[d1] = y[c];
-                            }
+                            for (int c = 0; c < 32; ++c, p += step)
+                                if (place >= 0) *p = y[c];
+                        } else {
+#pragma unroll
+                            for (int c = 0; c < 32; ++c, p += step)
+                                if (place >= 0 && ((stepped >> c) & 1u)) *p = y[c];
                         }
+                    };
+                    if (stepped) {
+                        put(d0);
+                        if (twice) put(d1);
                     }
                 }
             }
@@ -560,7 +561,7 @@ __global__ void psf_batch_pack(const GroupDev *__restrict__ groups, const SlotDe
 // sums of the slots' particle counts; a particle finds its slot by binary
 // search in shared memory.  Slots that did not advance this step (step limit
 // reached) are skipped.
-template <bool ALL_CENTRED>
+template <bool ALL_CENTRED, bool FACES>
 __global__ void __launch_bounds__(128, 5) psf_batch_trace(const GroupDev *__restrict__ groups,
                                                           const SlotDev *__restrict__ slots,
                                                           const long long *__restrict__ prefix, int n_slots)
@@ -576,7 +577,7 @@ __global__ void __launch_bounds__(128, 5) psf_batch_trace(const GroupDev *__rest
     size_t base = 0;
     TraceParams tp;
     uint64_t step = 0;
-    const float2 *pairs = nullptr;
+    const float *field = nullptr;
     const GroupDev *G = nullptr;
     for (long long gi = (long long)blockIdx.x * blockDim.x + threadIdx.x; gi < total; gi += stride) {
         if (cur < 0 || gi >= pre[cur + 1]) {
@@ -606,13 +607,16 @@ __global__ void __launch_bounds__(128, 5) psf_batch_trace(const GroupDev *__rest
             tp.rk4 = s.rk4;
             tp.seed = s.seed;
             step = s.step - 1ull;
-            pairs = G->pairs + (size_t)s.slot * 3 * (size_t)G->V;
+            field = G->field + (size_t)s.slot * (size_t)G->field_floats;
         }
         if (!live) continue;
         const size_t idx = base + (size_t)gi;
         float4 p = G->parts[idx];
-        if (ALL_CENTRED || G->grid.centered)
-            p = advance_particle<CentredBox>(p, G->grid, pairs, tp, step, G->perm, idx);
+        const float2 *pairs = reinterpret_cast<const float2 *>(field);
+        if (FACES)
+            p = advance_particle<CentredBox<FaceField>>(p, G->grid, field, tp, step, G->perm, idx);
+        else if (ALL_CENTRED || G->grid.centered)
+            p = advance_particle<CentredBox<PairField>>(p, G->grid, pairs, tp, step, G->perm, idx);
         else
             p = advance_particle<AnyBox>(p, G->grid, pairs, tp, step, G->perm, idx);
         G->parts[idx] = p;
@@ -731,22 +735,26 @@ int launch_batch_pack(const GroupDev *groups, const SlotDev *slots, int slot_glo
     return e == cudaSuccess ? PSF_OK : cuda_fail(e, "psf_batch_pack launch");
 }
 
-int batch_trace_grid(int num_sms)
+int batch_trace_grid(int num_sms, bool faces)
 {
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, psf_batch_trace<true>, 128, 0) != cudaSuccess || per_sm < 1)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+            &per_sm, faces ? psf_batch_trace<true, true> : psf_batch_trace<true, false>, 128, 0) != cudaSuccess ||
+        per_sm < 1)
         per_sm = 4;
     return num_sms * per_sm;
 }
 
 int launch_batch_trace(const GroupDev *groups, const SlotDev *slots, const long long *prefix, int n_slots, int grid,
-                       bool all_centred, cudaStream_t st)
+                       bool all_centred, bool faces, cudaStream_t st)
 {
     if (n_slots < 1 || n_slots > BATCH_MAX_ALL_SLOTS) return fail(PSF_ERR_INVALID, "slot count out of range");
-    if (all_centred)
-        psf_batch_trace<true><<<grid, 128, 0, st>>>(groups, slots, prefix, n_slots);
+    if (faces)
+        psf_batch_trace<true, true><<<grid, 128, 0, st>>>(groups, slots, prefix, n_slots);
+    else if (all_centred)
+        psf_batch_trace<true, false><<<grid, 128, 0, st>>>(groups, slots, prefix, n_slots);
     else
-        psf_batch_trace<false><<<grid, 128, 0, st>>>(groups, slots, prefix, n_slots);
+        psf_batch_trace<false, false><<<grid, 128, 0, st>>>(groups, slots, prefix, n_slots);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? PSF_OK : cuda_fail(e, "psf_batch_trace launch");
 }

@@ -51,9 +51,10 @@ struct HostGroup {
     uint16_t *W = nullptr;    // BF16 [2][bn][Nj]
     double *lam = nullptr, *w = nullptr, *force = nullptr, *dwpart = nullptr;
     float *wf = nullptr;
-    float2 *pairs = nullptr;
+    float *field = nullptr;      // [cap][field_floats], FaceField or PairField
+    int64_t field_floats = 0;
     std::vector<int32_t> faces_host, dst_host;  // for reading a slot's face field back
-    int32_t *pair_dst = nullptr;
+    int32_t *field_dst = nullptr;
     int64_t V = 0;
     CUtensorMap mapC{}, mapPhi{}, mapW{};
 };
@@ -143,7 +144,8 @@ struct psf_batch {
     int ksplit = 1;   // K ranges per contraction row tile
     int gemm_ctas = 148;
     int trace_ctas = 592;
-    bool all_centred = true;  // every basis has a centred box (GridDev::centered)
+    bool all_centred = true;   // every basis has a centred box (GridDev::centered)
+    bool face_field = false;   // the slots' fields are FaceFields (else PairFields)
     double tuned_ms = 0.0;
     psf::OrderBufs order{};
     int64_t pmax_all = 0;
@@ -196,6 +198,17 @@ struct psf_batch {
 
 namespace {
 
+// The slots' face fields hold every face once (FaceField) below so many
+// particles per voxel, counting the slots' capacities, and twice (PairField)
+// above.  Once halves what the reconstruction stores, and stores it in whole
+// sectors: 333 -> 165 us for 513 slots on three domains (N = 256), 68.6 -> 60.3
+// us for 64 slots of N = 384.  The tracer's gathers then take 24 loads instead
+// of 12, which costs it up to a fifth.  Whole steps, pairs against faces: 256
+// slots of N = 64 on 32^3 171 / 107 us at 0.12 particles per voxel, 255 / 218 at
+// 0.5, 366 / 349 at 1, 586 / 593 at 2; 128 slots of N = 256 129 / 111 at 0.25,
+// 210 / 213 at 1; 32 slots of N = 48 35.7 / 33.4 at 0.25, 56 / 59 at 1.
+constexpr double FACE_FIELD_DENSITY = 0.75;
+
 int upload_basis(psf_batch *B, HostGroup &G, const psf_batch_basis &bb)
 {
     const psf_basis_desc &b = bb.basis;
@@ -239,12 +252,22 @@ int upload_basis(psf_batch *B, HostGroup &G, const psf_batch_basis &bb)
     PSF_CHECK(B->alloc(&G.force, cap * N));
     PSF_CHECK(B->alloc(&G.dwpart, (size_t)N * G.a_tiles * 4 * psf::GEMM_MAX_KSPLIT * cap));
     G.faces_host.assign(b.active_faces, b.active_faces + G.F_act);
-    psf::face_pair_slots(G.grid, b.active_faces, G.F_act, G.dst_host);
-    PSF_CHECK(B->alloc(&G.pair_dst, G.dst_host.size()));
-    PSF_CUDA(cudaMemcpyAsync(G.pair_dst, G.dst_host.data(), G.dst_host.size() * 4, cudaMemcpyHostToDevice, st));
+    if (B->face_field) {
+        G.dst_host.resize((size_t)(2 * G.F_act));
+        for (int64_t r = 0; r < G.F_act; ++r) {
+            G.dst_host[(size_t)(2 * r)] = b.active_faces[r];
+            G.dst_host[(size_t)(2 * r + 1)] = -1;
+        }
+        G.field_floats = G.n_faces;
+    } else {
+        psf::face_pair_slots(G.grid, b.active_faces, G.F_act, G.dst_host);
+        G.field_floats = 6 * G.V;
+    }
+    PSF_CHECK(B->alloc(&G.field_dst, G.dst_host.size()));
+    PSF_CUDA(cudaMemcpyAsync(G.field_dst, G.dst_host.data(), G.dst_host.size() * 4, cudaMemcpyHostToDevice, st));
     PSF_CUDA(cudaStreamSynchronize(st));
-    PSF_CHECK(B->alloc(&G.pairs, cap * (size_t)(3 * G.V)));
-    PSF_CUDA(cudaMemsetAsync(G.pairs, 0, cap * (size_t)(3 * G.V) * sizeof(float2), st));
+    PSF_CHECK(B->alloc(&G.field, cap * (size_t)G.field_floats));
+    PSF_CUDA(cudaMemsetAsync(G.field, 0, cap * (size_t)G.field_floats * sizeof(float), st));
     PSF_CUDA(cudaMemsetAsync(G.W, 0, (size_t)2 * G.bn * G.Nj * 2, st));
     PSF_CUDA(cudaMemsetAsync(G.w, 0, cap * N * 8, st));
     PSF_CUDA(cudaMemsetAsync(G.force, 0, cap * N * 8, st));
@@ -320,9 +343,9 @@ void fill_gemm_args(psf_batch *B)
         y.n_rows = (int)G.F_act;
         y.ldw = G.N;
         y.n_faces = G.n_faces;
-        y.pair_dst = G.pair_dst;
-        y.pairs = reinterpret_cast<float *>(G.pairs);
-        y.pair_floats = 6 * G.V;
+        y.field_dst = G.field_dst;
+        y.field = G.field;
+        y.field_floats = G.field_floats;
         y.slot_of = B->d_slots + G.slot_base;
         c.r_tiles += y.tiles;
     }
@@ -340,7 +363,6 @@ int upload_tables(psf_batch *B)
         const HostGroup &G = B->groups[gi];
         psf::GroupDev &d = gd[gi];
         d.grid = psf::make_grid_dev(G.grid);
-        if (!d.grid.centered) B->all_centred = false;
         d.N = G.N;
         d.Nj = G.Nj;
         d.cap = G.cap;
@@ -356,7 +378,8 @@ int upload_tables(psf_batch *B)
         d.lam = G.lam;
         d.dwpart = G.dwpart;
         d.W = G.W;
-        d.pairs = G.pairs;
+        d.field = G.field;
+        d.field_floats = G.field_floats;
         d.V = G.V;
         d.parts = B->pool_parts;
         d.perm = B->pool_perm;
@@ -497,7 +520,7 @@ int launch_step(psf_batch *B, cudaStream_t st)
 {
     PSF_CHECK(launch_tc_part(B, st, B->use_fused));
     PSF_CHECK(psf::launch_batch_trace(B->d_groups, B->d_slots, B->d_prefix, B->n_slots(), B->trace_ctas,
-                                      B->all_centred, st));
+                                      B->all_centred, B->face_field, st));
     return PSF_OK;
 }
 
@@ -606,6 +629,18 @@ int psf_batch_create(const psf_batch_config *cfg, int device, psf_batch **out)
     if ((e = cudaMemsetAsync(B->d_err, 0, sizeof(int), B->stream)) != cudaSuccess)
         return bail(psf::cuda_fail(e, "cudaMemset"));
 
+    // Field form: see FACE_FIELD_DENSITY.
+    {
+        double voxels = 0.0, particles = 0.0;
+        for (int i = 0; i < cfg->n_bases; ++i) {
+            const psf_grid &g = cfg->bases[i].basis.grid;
+            voxels += (double)cfg->bases[i].slots * g.dims[0] * g.dims[1] * g.dims[2];
+            particles += (double)cfg->bases[i].slots * (double)cfg->bases[i].max_particles;
+            if (!psf::make_grid_dev(g).centered) B->all_centred = false;
+        }
+        B->face_field = B->all_centred && particles < FACE_FIELD_DENSITY * voxels;
+    }
+
     int slot_base = 0;
     B->groups.resize((size_t)cfg->n_bases);
     try {
@@ -666,7 +701,7 @@ int psf_batch_create(const psf_batch_config *cfg, int device, psf_batch **out)
     }
     fill_gemm_args(B);
     if ((rc = upload_tables(B)) != PSF_OK || (rc = upload_prefix(B)) != PSF_OK) return bail(rc);
-    B->trace_ctas = psf::batch_trace_grid(B->num_sms);
+    B->trace_ctas = psf::batch_trace_grid(B->num_sms, B->face_field);
     B->gemm_ctas = cfg->gemm_ctas > 0 ? cfg->gemm_ctas : B->num_sms;
     if (cfg->gemm_columns != 0) {
         B->bn_max = cfg->gemm_columns;
@@ -952,15 +987,14 @@ int psf_batch_get_velocity(psf_batch *B, int32_t basis, int32_t slot, float *u, 
     if (!u) return fail(PSF_ERR_INVALID, "null argument");
     if (n_faces != G.n_faces) return fail(PSF_ERR_INVALID, "n_faces must equal the grid's face count");
     PSF_CUDA(cudaSetDevice(B->device));
-    // The slot's field lives in its per-voxel face pairs; every active face is
-    // stored in both adjacent voxels, wall faces are zero.
+    // Every active face has a place in the slot's field; wall faces are zero.
     std::vector<float> pf;
     try {
-        pf.resize((size_t)(6 * G.V));
+        pf.resize((size_t)G.field_floats);
     } catch (const std::bad_alloc &) {
         return fail(PSF_ERR_NOMEM, "host staging allocation failed");
     }
-    PSF_CUDA(cudaMemcpyAsync(pf.data(), G.pairs + (size_t)slot * 3 * G.V, pf.size() * 4, cudaMemcpyDeviceToHost,
+    PSF_CUDA(cudaMemcpyAsync(pf.data(), G.field + (size_t)slot * (size_t)G.field_floats, pf.size() * 4, cudaMemcpyDeviceToHost,
                              B->stream));
     PSF_CUDA(cudaStreamSynchronize(B->stream));
     std::fill(u, u + n_faces, 0.f);
@@ -1008,7 +1042,7 @@ static int profile(psf_batch *B, double *kernel_ms, int32_t n, bool fused)
     }
     if (rc == PSF_OK)
         rc = psf::launch_batch_trace(B->d_groups, B->d_slots, B->d_prefix, B->n_slots(), B->trace_ctas,
-                                      B->all_centred, st);
+                                      B->all_centred, B->face_field, st);
     cudaEventRecord(ev[nk], st);
     cudaError_t e = cudaStreamSynchronize(st);
     if (rc == PSF_OK && e != cudaSuccess) rc = psf::cuda_fail(e, "profiled step");

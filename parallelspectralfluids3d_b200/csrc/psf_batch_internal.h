@@ -14,7 +14,9 @@ namespace psf {
 constexpr int BATCH_MAX_GROUPS = 6;   // distinct bases in one batch
 constexpr int BATCH_MAX_SLOTS = 256;  // instance slots per basis (one MMA N tile)
 constexpr int BATCH_MAX_ALL_SLOTS = BATCH_MAX_GROUPS * BATCH_MAX_SLOTS;
-constexpr int GEMM_THREADS = 192;     // warp 0 TMA, warp 1 MMA, warps 2-5 epilogue
+constexpr int EPI_WARPS = 8;          // epilogue: two warps per TMEM lane quarter
+constexpr int EPI_THREADS = 32 * EPI_WARPS;
+constexpr int GEMM_THREADS = 64 + EPI_THREADS;  // warp 0 TMA, warp 1 MMA, warps 2-9 epilogue
 constexpr int GEMM_MAX_KSPLIT = 4;
 
 // One basis inside a GEMM launch: A operand (C or Phi) and B operand (the
@@ -39,10 +41,10 @@ struct alignas(64) GemmGroup {
     double *dwpart;         // contraction: partials [k][nparts (a-tile, K range, warp)][slot]
     int nparts;             // contraction: partials per (slot, k)
     long long n_faces;
-    const int32_t *pair_dst;  // reconstruction: [n_rows][2] float slots in a slot's face pairs
-    float *pairs;           // reconstruction: per-voxel face pairs [cap][3V] (float2)
-    long long pair_floats;  // 6V: floats per slot in pairs
-    const SlotDev *slot_of; // reconstruction: the group's slots (column b is slot_of[b]); pairs are
+    const int32_t *field_dst;  // reconstruction: [n_rows][2] places of a face in a slot's field (-1: none)
+    float *field;           // reconstruction: the slots' face fields, FaceField or PairField (psf_device.cuh)
+    long long field_floats; // floats per slot in field
+    const SlotDev *slot_of; // reconstruction: the group's slots (column b is slot_of[b]); fields are
                             // written only for slots that stepped (the tracer reads no others)
 };
 
@@ -97,7 +99,8 @@ struct GroupDev {
     const double *lam;    // [N]
     double *dwpart;       // see GemmGroup
     uint16_t *W;          // BF16 [2][bn][Nj]
-    float2 *pairs;        // [cap][3V] per-voxel face pairs of each slot
+    float *field;         // [cap][field_floats] face field of each slot
+    long long field_floats;
     long long V;
     float4 *parts;        // particle pool (all slots of the batch)
     int32_t *perm;        // caller index of each pooled particle
@@ -112,9 +115,9 @@ int max_fused_grid(int bn_max, int num_sms);
 int launch_batch_state(const GroupDev *groups, SlotDev *slots, int n_slots, cudaStream_t st);
 // prefix[s] = particles of slots 0..s-1 (occupied slots only); n_slots + 1 entries.
 int launch_batch_trace(const GroupDev *groups, const SlotDev *slots, const long long *prefix, int n_slots, int grid,
-                       bool all_centred, cudaStream_t st);
+                       bool all_centred, bool faces, cudaStream_t st);
 int launch_batch_pack(const GroupDev *groups, const SlotDev *slots, int slot_global, cudaStream_t st);
-int batch_trace_grid(int num_sms);
+int batch_trace_grid(int num_sms, bool faces);
 
 // Host helpers.
 int encode_tensor_map(CUtensorMap *map, void *base, int rank, const uint64_t *dims, const uint64_t *strides_bytes,

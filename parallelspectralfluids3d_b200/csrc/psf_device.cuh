@@ -175,6 +175,7 @@ __device__ __forceinline__ float3 interpolate(const CellCache &c, const float3 &
 // `c` carries the last gathered cell, and the samples are loaded again only
 // when the position lies in another cell.
 struct AnyBox {
+    using Ptr = const float2 *__restrict__;
     CellCache c;
     bool have = false;
     __device__ __forceinline__ float3 velocity(const GridDev &g, const float2 *__restrict__ pairs, float px, float py,
@@ -191,6 +192,50 @@ struct AnyBox {
         }
         return interpolate(c, make_float3((px - g.mn[0]) * g.inv_h, (py - g.mn[1]) * g.inv_h,
                                           (pz - g.mn[2]) * g.inv_h));
+    }
+};
+
+// The two forms of a face field and the two faces of voxel (x, y, z) along an
+// axis, with the tracer's signs.  PairField holds them side by side, every
+// face twice: one load.  FaceField is the reference's face numbering, every
+// face once: two loads, half the memory.
+struct PairField {
+    using Ptr = const float2 *__restrict__;
+    Ptr px, py, pz;
+    uint32_t nx, nxy;
+    __device__ __forceinline__ PairField(const GridDev &g, Ptr p) : px(p), nx((uint32_t)g.nx)
+    {
+        nxy = nx * (uint32_t)g.ny;
+        py = p + nxy * (uint32_t)g.nz;
+        pz = p + 2 * (size_t)(nxy * (uint32_t)g.nz);
+    }
+    __device__ __forceinline__ float2 x(uint32_t i, uint32_t j, uint32_t k) const { return __ldg(px + (k * nxy + j * nx + i)); }
+    __device__ __forceinline__ float2 y(uint32_t i, uint32_t j, uint32_t k) const { return __ldg(py + (k * nxy + j * nx + i)); }
+    __device__ __forceinline__ float2 z(uint32_t i, uint32_t j, uint32_t k) const { return __ldg(pz + (k * nxy + j * nx + i)); }
+};
+
+struct FaceField {
+    using Ptr = const float *__restrict__;
+    Ptr px, py, pz;
+    uint32_t nx, ny, nxy;
+    __device__ __forceinline__ FaceField(const GridDev &g, Ptr u)
+        : px(u + g.xoff), py(u + g.yoff), pz(u), nx((uint32_t)g.nx), ny((uint32_t)g.ny), nxy((uint32_t)(g.nx * g.ny))
+    {
+    }
+    __device__ __forceinline__ float2 x(uint32_t i, uint32_t j, uint32_t k) const
+    {
+        const uint32_t f = (k * ny + j) * (nx + 1) + i;
+        return make_float2(__ldg(px + f), __ldg(px + f + 1));
+    }
+    __device__ __forceinline__ float2 y(uint32_t i, uint32_t j, uint32_t k) const
+    {
+        const uint32_t f = k * (nxy + nx) + j * nx + i;
+        return make_float2(__ldg(py + f), __ldg(py + f + nx));
+    }
+    __device__ __forceinline__ float2 z(uint32_t i, uint32_t j, uint32_t k) const
+    {
+        const uint32_t f = k * nxy + j * nx + i;
+        return make_float2(__ldg(pz + f), __ldg(pz + f + nxy));
     }
 };
 
@@ -228,14 +273,14 @@ struct Trilinear {
 // places cost more in the repeated gathers) and the 512-slot reconstruction
 // 353 against 302 us; storing every face once (24 loads of 4 bytes) was slower
 // at every density.
+template <class Field>
 struct CentredBox {
     float ox, oy, oz;     // whole-cell origin
     float sx, sy, sz;     // half-shifted origin
     Trilinear x, y, z;
     bool have = false;
 
-    __device__ __forceinline__ void gather(const GridDev &g, const float2 *__restrict__ pairs, float qx, float qy,
-                                           float qz)
+    __device__ __forceinline__ void gather(const GridDev &g, typename Field::Ptr u, float qx, float qy, float qz)
     {
         const int kx = clampi(__float2int_rd(2.0f * (qx * g.inv_h)), 0, 2 * g.nx - 1);
         const int ky = clampi(__float2int_rd(2.0f * (qy * g.inv_h)), 0, 2 * g.ny - 1);
@@ -248,19 +293,13 @@ struct CentredBox {
         sx = (float)xr + 0.5f;
         sy = (float)yr + 0.5f;
         sz = (float)zr + 0.5f;
-        const int xM = max(xr, 0), xP = min(xr + 1, g.nx - 1);
-        const uint32_t nx = (uint32_t)g.nx, nxy = (uint32_t)(g.nx * g.ny), V = nxy * (uint32_t)g.nz;
-        const uint32_t yM = (uint32_t)max(yr, 0) * nx, yP = (uint32_t)min(yr + 1, g.ny - 1) * nx;
-        const uint32_t zM = (uint32_t)max(zr, 0) * nxy, zP = (uint32_t)min(zr + 1, g.nz - 1) * nxy;
-        const uint32_t yW = (uint32_t)yO * nx, zW = (uint32_t)zO * nxy;
-        const float2 *__restrict__ py = pairs + V;
-        const float2 *__restrict__ pz = pairs + 2 * (size_t)V;
-        const float2 x00 = __ldg(pairs + (zM + yM + xO)), x10 = __ldg(pairs + (zM + yP + xO));
-        const float2 x01 = __ldg(pairs + (zP + yM + xO)), x11 = __ldg(pairs + (zP + yP + xO));
-        const float2 y00 = __ldg(py + (zM + yW + xM)), y10 = __ldg(py + (zM + yW + xP));
-        const float2 y01 = __ldg(py + (zP + yW + xM)), y11 = __ldg(py + (zP + yW + xP));
-        const float2 z00 = __ldg(pz + (zW + yM + xM)), z01 = __ldg(pz + (zW + yP + xM));
-        const float2 z10 = __ldg(pz + (zW + yM + xP)), z11 = __ldg(pz + (zW + yP + xP));
+        const uint32_t xM = (uint32_t)max(xr, 0), xP = (uint32_t)min(xr + 1, g.nx - 1);
+        const uint32_t yM = (uint32_t)max(yr, 0), yP = (uint32_t)min(yr + 1, g.ny - 1);
+        const uint32_t zM = (uint32_t)max(zr, 0), zP = (uint32_t)min(zr + 1, g.nz - 1);
+        const Field f(g, u);
+        const float2 x00 = f.x(xO, yM, zM), x10 = f.x(xO, yP, zM), x01 = f.x(xO, yM, zP), x11 = f.x(xO, yP, zP);
+        const float2 y00 = f.y(xM, yO, zM), y10 = f.y(xP, yO, zM), y01 = f.y(xM, yO, zP), y11 = f.y(xP, yO, zP);
+        const float2 z00 = f.z(xM, yM, zO), z01 = f.z(xM, yP, zO), z10 = f.z(xP, yM, zO), z11 = f.z(xP, yP, zO);
         auto plane = [](float v, float vy, float vx, float vxy, float &o, float &dy, float &dx, float &dxy) {
             o = v;
             dy = vy - v;
@@ -280,18 +319,17 @@ struct CentredBox {
         return __float_as_uint(fminf(a, b)) <= 0x3F000000u;  // [0, 1/2]
     }
 
-    __device__ __forceinline__ float3 velocity(const GridDev &g, const float2 *__restrict__ pairs, float px, float py,
-                                               float pz)
+    __device__ __forceinline__ float3 velocity(const GridDev &g, typename Field::Ptr u, float px, float py, float pz)
     {
         const float qx = px - g.mn[0], qy = py - g.mn[1], qz = pz - g.mn[2];
         if (!have) {
-            gather(g, pairs, qx, qy, qz);
+            gather(g, u, qx, qy, qz);
             have = true;
         } else {
             const bool same = inside(fmaf(qx, g.inv_h, -ox), fmaf(qx, g.inv_h, -sx)) &&
                               inside(fmaf(qy, g.inv_h, -oy), fmaf(qy, g.inv_h, -sy)) &&
                               inside(fmaf(qz, g.inv_h, -oz), fmaf(qz, g.inv_h, -sz));
-            if (!same) gather(g, pairs, qx, qy, qz);
+            if (!same) gather(g, u, qx, qy, qz);
         }
         const float ax = fmaf(qx, g.inv_h, -ox), ay = fmaf(qy, g.inv_h, -oy), az = fmaf(qz, g.inv_h, -oz);
         const float bx = fmaf(qx, g.inv_h, -sx), by = fmaf(qy, g.inv_h, -sy), bz = fmaf(qz, g.inv_h, -sz);
@@ -321,8 +359,8 @@ __device__ __forceinline__ float div6(float x)
 // generator keyed by the caller-order index `perm[idx]` when the lifetime ran
 // out (read only then).  `step` is the index of the step being taken (0 for
 // the first).
-template <class Box>
-__device__ __forceinline__ float4 advance_particle(float4 p, const GridDev &g, const float2 *__restrict__ u,
+template <class Box, class Ptr>
+__device__ __forceinline__ float4 advance_particle(float4 p, const GridDev &g, Ptr u,
                                                    const TraceParams &tp, uint64_t step,
                                                    const int32_t *__restrict__ perm, size_t idx)
 {
