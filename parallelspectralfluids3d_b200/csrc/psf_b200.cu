@@ -50,14 +50,6 @@ int cuda_fail(cudaError_t e, const char *what)
                 std::string(what) + ": " + cudaGetErrorString(e));
 }
 
-// --------------------------------------------- programmatic dependent launch
-// The three step kernels run back to back in one stream.  Each one loads only
-// constant data (C rows, Phi tiles, face maps) before griddepcontrol.wait, and
-// lets its own dependents launch only after that wait: at most two kernels
-// are in flight, and the second never reads what the first is still writing.
-__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
-__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
-
 // ------------------------------------------------------- 1. contraction
 // Block b handles mode k = b / S and row slice s = b % S of C_k.  Lane l of a
 // warp owns columns [4l + 128c, 4l + 128c + 4) for c < CH; warps walk rows a.
@@ -378,29 +370,10 @@ int launch_unorder_particles(const PlainDev &d, const OrderBufs &o, cudaStream_t
 }
 
 // ------------------------------------------------------------- launchers
-// Launch configuration of a step kernel that may start while the previous
-// kernel in the stream finishes (programmatic stream serialisation).
-struct PdlLaunch {
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
-    PdlLaunch(unsigned grid, unsigned block, cudaStream_t st)
-    {
-        cfg.gridDim = dim3(grid);
-        cfg.blockDim = dim3(block);
-        cfg.dynamicSmemBytes = 0;
-        cfg.stream = st;
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-    }
-};
-
 int launch_contract_state(const PlainDev &d, cudaStream_t st, bool after_kernel)
 {
     const int CH = (d.Np + 127) / 128;
-    PdlLaunch L((unsigned)(d.N * d.S), 256, st);
-    if (!after_kernel) L.cfg.numAttrs = 0;
+    PdlLaunch L((unsigned)(d.N * d.S), 256, st, after_kernel);
     cudaError_t e = cudaSuccess;
 #define PSF_CASE(n)                                                                                             \
     case n:                                                                                                     \
@@ -427,8 +400,7 @@ int launch_contract_state(const PlainDev &d, cudaStream_t st, bool after_kernel)
 int launch_reconstruct(const PlainDev &d, cudaStream_t st, bool after_kernel)
 {
     const long long blocks = (d.n_active + 127) / 128;
-    PdlLaunch L((unsigned)blocks, 256, st);
-    if (!after_kernel) L.cfg.numAttrs = 0;
+    PdlLaunch L((unsigned)blocks, 256, st, after_kernel);
     cudaError_t e = cudaLaunchKernelEx(&L.cfg, psf_reconstruct, (const float *)d.phiT, (long long)d.ldp,
                                        (const int32_t *)d.faces, (long long)d.n_active, (int)d.N, (const double *)d.w,
                                        d.u, reinterpret_cast<float *>(d.pairs), (const int32_t *)d.pair_dst);
@@ -449,8 +421,7 @@ int launch_trace(const PlainDev &d, cudaStream_t st, bool after_kernel)
     if (d.P == 0) return PSF_OK;
     const long long blocks =
         std::min<long long>((d.P + TRACE_THREADS - 1) / TRACE_THREADS, std::max(1, d.trace_blocks));
-    PdlLaunch L((unsigned)blocks, TRACE_THREADS, st);
-    if (!after_kernel) L.cfg.numAttrs = 0;
+    PdlLaunch L((unsigned)blocks, TRACE_THREADS, st, after_kernel);
     cudaError_t e = cudaLaunchKernelEx(&L.cfg, d.grid.centered ? psf_trace<CentredBox<PairField>> : psf_trace<AnyBox>, d.parts, (long long)d.P, (const int32_t *)d.perm,
                                        d.trace_pairs, d.grid, d.tp, d.trace_ctr);
     return e == cudaSuccess ? PSF_OK : cuda_fail(e, "psf_trace launch");

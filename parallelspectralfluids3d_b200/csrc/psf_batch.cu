@@ -265,13 +265,19 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) psf_batch_step_tc(const __gri
             uint32_t last_parity[STAGES];
             bool issued[STAGES];
             for (int s = 0; s < STAGES; ++s) issued[s] = false;
-            // Reconstruction stages whose W load waits for the state update.
+            // Stages whose W load waits for the state update (in this launch or
+            // in the kernel before): their C or Phi tiles load meanwhile.
             int pend_stage[STAGES], pend_kc[STAGES], pend_t[STAGES];
             int npend = 0;
-            bool w_ok = MODE != 2;
+            bool w_ok = false;
             bool ok = true;
             auto flush = [&]() -> bool {
-                if (!mbar_wait(wready, 0u, err, ERR_WAIT_STATE)) return false;
+                if (MODE == 2) {
+                    if (!mbar_wait(wready, 0u, err, ERR_WAIT_STATE)) return false;
+                } else {
+                    grid_dependency_wait();
+                    launch_dependents();
+                }
                 for (int i = 0; i < npend; ++i) {
                     bool rc;
                     int lt;
@@ -380,6 +386,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) psf_batch_step_tc(const __gri
         const int row = q * 32 + lane;
         int abuf = 0;
         uint32_t aphase = 0;
+        if (MODE != 2) grid_dependency_wait();
         if (MODE == 2) {
             // Every slot's state update (one CTA per slot), then a grid
             // barrier before any coefficient (W) load of the sweep.
@@ -503,6 +510,8 @@ __global__ void __launch_bounds__(256) psf_batch_state(const GroupDev *__restric
 {
     __shared__ double red[8];
     __shared__ double wnew[PSF_MAX_MODES];
+    grid_dependency_wait();
+    launch_dependents();
     SlotDev &s = slots[blockIdx.x];
     if (!s.active) return;
     if (s.target != 0ull && s.step >= s.target) {
@@ -569,6 +578,8 @@ __global__ void __launch_bounds__(128, 5) psf_batch_trace(const GroupDev *__rest
     __shared__ long long pre[BATCH_MAX_ALL_SLOTS + 1];
     for (int i = threadIdx.x; i <= n_slots; i += blockDim.x) pre[i] = prefix[i];
     __syncthreads();
+    grid_dependency_wait();
+    launch_dependents();
     const long long total = pre[n_slots];
     const long long stride = (long long)gridDim.x * blockDim.x;
     // Parameters of the slot the thread is in, reloaded only when it changes.
@@ -635,7 +646,7 @@ int batch_gemm_smem_bytes(int bn_max)
 }
 
 template <int BN, int MODE>
-static int launch_tc_t(const StepArgs &args, int grid, cudaStream_t st)
+static int launch_tc_t(const StepArgs &args, int grid, cudaStream_t st, bool after_kernel)
 {
     // The shared-memory limit is a per-device attribute of the kernel.
     static unsigned long long configured = 0;
@@ -649,33 +660,29 @@ static int launch_tc_t(const StepArgs &args, int grid, cudaStream_t st)
         if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(psf_batch_step_tc)");
         configured |= bit;
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(GEMM_THREADS);
-    cfg.dynamicSmemBytes = GemmCfg<BN>::SMEM;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = MODE == 2 ? 1 : 0;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, psf_batch_step_tc<BN, MODE>, args);
+    PdlLaunch L((unsigned)grid, GEMM_THREADS, st, after_kernel && MODE != 2, GemmCfg<BN>::SMEM);
+    if (MODE == 2) {
+        L.attr[0].id = cudaLaunchAttributeCooperative;
+        L.attr[0].val.cooperative = 1;
+        L.cfg.numAttrs = 1;
+    }
+    e = cudaLaunchKernelEx(&L.cfg, psf_batch_step_tc<BN, MODE>, args);
     if (e != cudaSuccess) return cuda_fail(e, "psf_batch_step_tc launch");
     return PSF_OK;
 }
 
 template <int MODE>
-static int launch_tc_mode(const StepArgs &args, int bn_max, int grid, cudaStream_t st)
+static int launch_tc_mode(const StepArgs &args, int bn_max, int grid, cudaStream_t st, bool after_kernel)
 {
     switch (bn_max) {
-    case 64: return launch_tc_t<64, MODE>(args, grid, st);
-    case 128: return launch_tc_t<128, MODE>(args, grid, st);
-    case 256: return launch_tc_t<256, MODE>(args, grid, st);
+    case 64: return launch_tc_t<64, MODE>(args, grid, st, after_kernel);
+    case 128: return launch_tc_t<128, MODE>(args, grid, st, after_kernel);
+    case 256: return launch_tc_t<256, MODE>(args, grid, st, after_kernel);
     }
     return fail(PSF_ERR_UNSUPPORTED, "GEMM variant must have 64, 128 or 256 columns");
 }
 
-int launch_batch_step_tc(const StepArgs &args, int bn_max, int grid, cudaStream_t st)
+int launch_batch_step_tc(const StepArgs &args, int bn_max, int grid, cudaStream_t st, bool after_kernel)
 {
     const int total = args.c_tiles + args.r_tiles;
     if (total <= 0 && !args.fused) return PSF_OK;
@@ -686,9 +693,9 @@ int launch_batch_step_tc(const StepArgs &args, int bn_max, int grid, cudaStream_
         if (used && (args.g[g].bn > bn_max || args.g[g].bn % 16 != 0 || args.g[g].bn < 16))
             return fail(PSF_ERR_INVALID, "GEMM group N tile does not fit the kernel variant");
     }
-    if (args.fused) return launch_tc_mode<2>(args, bn_max, grid, st);
-    if (args.r_tiles == 0) return launch_tc_mode<0>(args, bn_max, grid, st);
-    if (args.c_tiles == 0) return launch_tc_mode<1>(args, bn_max, grid, st);
+    if (args.fused) return launch_tc_mode<2>(args, bn_max, grid, st, after_kernel);
+    if (args.r_tiles == 0) return launch_tc_mode<0>(args, bn_max, grid, st, after_kernel);
+    if (args.c_tiles == 0) return launch_tc_mode<1>(args, bn_max, grid, st, after_kernel);
     return fail(PSF_ERR_INVALID, "an unfused launch runs either contraction or reconstruction units");
 }
 
@@ -720,11 +727,11 @@ int max_fused_grid(int bn_max, int num_sms)
     return per_sm * num_sms;
 }
 
-int launch_batch_state(const GroupDev *groups, SlotDev *slots, int n_slots, cudaStream_t st)
+int launch_batch_state(const GroupDev *groups, SlotDev *slots, int n_slots, cudaStream_t st, bool after_kernel)
 {
     if (n_slots <= 0) return PSF_OK;
-    psf_batch_state<<<n_slots, 256, 0, st>>>(groups, slots);
-    cudaError_t e = cudaGetLastError();
+    PdlLaunch L((unsigned)n_slots, 256, st, after_kernel);
+    cudaError_t e = cudaLaunchKernelEx(&L.cfg, psf_batch_state, groups, slots);
     return e == cudaSuccess ? PSF_OK : cuda_fail(e, "psf_batch_state launch");
 }
 
@@ -746,16 +753,15 @@ int batch_trace_grid(int num_sms, bool faces)
 }
 
 int launch_batch_trace(const GroupDev *groups, const SlotDev *slots, const long long *prefix, int n_slots, int grid,
-                       bool all_centred, bool faces, cudaStream_t st)
+                       bool all_centred, bool faces, cudaStream_t st, bool after_kernel)
 {
     if (n_slots < 1 || n_slots > BATCH_MAX_ALL_SLOTS) return fail(PSF_ERR_INVALID, "slot count out of range");
-    if (faces)
-        psf_batch_trace<true, true><<<grid, 128, 0, st>>>(groups, slots, prefix, n_slots);
-    else if (all_centred)
-        psf_batch_trace<true, false><<<grid, 128, 0, st>>>(groups, slots, prefix, n_slots);
-    else
-        psf_batch_trace<false, false><<<grid, 128, 0, st>>>(groups, slots, prefix, n_slots);
-    cudaError_t e = cudaGetLastError();
+    PdlLaunch L((unsigned)grid, 128, st, after_kernel);
+    cudaError_t e = cudaLaunchKernelEx(&L.cfg,
+                                       faces         ? psf_batch_trace<true, true>
+                                       : all_centred ? psf_batch_trace<true, false>
+                                                     : psf_batch_trace<false, false>,
+                                       groups, slots, prefix, n_slots);
     return e == cudaSuccess ? PSF_OK : cuda_fail(e, "psf_batch_trace launch");
 }
 

@@ -110,12 +110,14 @@ struct GroupDev {
 // Launchers (psf_batch.cu).  `bn_max` selects the kernel variant (64, 128 or
 // 256 MMA columns per accumulator); `grid` the number of persistent CTAs.
 int batch_gemm_smem_bytes(int bn_max);
-int launch_batch_step_tc(const StepArgs &args, int bn_max, int grid, cudaStream_t st);
+// `after_kernel`: the launch directly follows a kernel in the stream and may
+// start during that kernel's tail (programmatic dependent launch).
+int launch_batch_step_tc(const StepArgs &args, int bn_max, int grid, cudaStream_t st, bool after_kernel = false);
 int max_fused_grid(int bn_max, int num_sms);
-int launch_batch_state(const GroupDev *groups, SlotDev *slots, int n_slots, cudaStream_t st);
+int launch_batch_state(const GroupDev *groups, SlotDev *slots, int n_slots, cudaStream_t st, bool after_kernel = false);
 // prefix[s] = particles of slots 0..s-1 (occupied slots only); n_slots + 1 entries.
 int launch_batch_trace(const GroupDev *groups, const SlotDev *slots, const long long *prefix, int n_slots, int grid,
-                       bool all_centred, bool faces, cudaStream_t st);
+                       bool all_centred, bool faces, cudaStream_t st, bool after_kernel = false);
 int launch_batch_pack(const GroupDev *groups, const SlotDev *slots, int slot_global, cudaStream_t st);
 int batch_trace_grid(int num_sms, bool faces);
 

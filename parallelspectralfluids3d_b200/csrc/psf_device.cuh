@@ -12,6 +12,33 @@
 
 namespace psf {
 
+// --------------------------------------------- programmatic dependent launch
+// The kernels of a step run back to back in one stream (or one branch of a
+// graph).  Each one touches only constant data (C, Phi, face maps, prefix
+// sums) before griddepcontrol.wait, and lets its own dependents launch only
+// after that wait: at most two kernels are in flight, and the second never
+// reads what the first is still writing.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+
+// Launch configuration of a kernel that may start while the previous kernel in
+// the stream finishes (programmatic stream serialisation), if `after_kernel`.
+struct PdlLaunch {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    PdlLaunch(unsigned grid, unsigned block, cudaStream_t st, bool after_kernel, size_t smem = 0)
+    {
+        cfg.gridDim = dim3(grid);
+        cfg.blockDim = dim3(block);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = after_kernel ? 1 : 0;
+    }
+};
+
 // ---------------------------------------------------------------- helpers
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return min(max(v, lo), hi); }
 // glm::mix(x, y, a) = x (1 - a) + y a, evaluated as x + a (y - x) (one FMA).
