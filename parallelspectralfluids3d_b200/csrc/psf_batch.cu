@@ -565,6 +565,23 @@ __global__ void psf_batch_pack(const GroupDev *__restrict__ groups, const SlotDe
     }
 }
 
+// ----------------------------------------------------------------- read-back
+__global__ void psf_batch_gather_states(const ReadJob *__restrict__ jobs, double *__restrict__ w_out)
+{
+    const ReadJob &j = jobs[blockIdx.x];
+    for (int i = threadIdx.x; i < j.n_w; i += blockDim.x) w_out[j.w_at + i] = j.w[i];
+}
+
+// A grid row per slot.  A slot by itself is a launch of a few microseconds that
+// moves a few hundred KB; together they run at the memory's rate.
+__global__ void psf_batch_unorder(const ReadJob *__restrict__ jobs, const float4 *__restrict__ pool,
+                                  const int32_t *__restrict__ perm, float4 *__restrict__ stage)
+{
+    const ReadJob &j = jobs[blockIdx.y];
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < j.n_parts; i += gridDim.x * blockDim.x)
+        stage[j.stage + perm[j.poff + i]] = pool[j.poff + i];
+}
+
 // ------------------------------------------------------------------ tracer
 // Every occupied slot's particles form one index space through the prefix
 // sums of the slots' particle counts; a particle finds its slot by binary
@@ -740,6 +757,24 @@ int launch_batch_pack(const GroupDev *groups, const SlotDev *slots, int slot_glo
     psf_batch_pack<<<1, 256, 0, st>>>(groups, slots, slot_global);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? PSF_OK : cuda_fail(e, "psf_batch_pack launch");
+}
+
+int launch_batch_gather_states(const ReadJob *jobs, int n, double *w_out, cudaStream_t st)
+{
+    if (n <= 0) return PSF_OK;
+    psf_batch_gather_states<<<n, 128, 0, st>>>(jobs, w_out);
+    cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? PSF_OK : cuda_fail(e, "psf_batch_gather_states launch");
+}
+
+int launch_batch_unorder(const ReadJob *jobs, int n, int max_parts, const float4 *pool, const int32_t *perm,
+                         float4 *stage, cudaStream_t st)
+{
+    if (n <= 0 || max_parts <= 0) return PSF_OK;
+    const dim3 grid((unsigned)std::min(256, (max_parts + 255) / 256), (unsigned)n);
+    psf_batch_unorder<<<grid, 256, 0, st>>>(jobs, pool, perm, stage);
+    cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? PSF_OK : cuda_fail(e, "psf_batch_unorder launch");
 }
 
 int batch_trace_grid(int num_sms, bool faces)

@@ -15,6 +15,7 @@
 #include <map>
 #include <new>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "psf_b200.h"
@@ -156,6 +157,12 @@ struct psf_batch {
     std::vector<int64_t> slot_units;  // pool units held by each slot
     int64_t bytes = 0;
     std::vector<void *> allocs;
+    // Grouped reads (psf_batch_read_instances): job table, gathered states with
+    // a pinned copy, and staging for READ_STAGE particles (or the largest slot).
+    psf::ReadJob *read_jobs = nullptr;
+    double *read_w = nullptr, *read_w_host = nullptr;
+    int64_t read_jobs_cap = 0, read_w_cap = 0, read_host_cap = 0, read_stage_cap = 0;
+    float4 *read_stage = nullptr;
     // Reads of slots that the queued steps do not touch (psf::batch_read_frozen):
     // a second stream and pinned host buffers for one slot's particles.
     cudaStream_t side = nullptr;
@@ -169,6 +176,8 @@ struct psf_batch {
     {
         drop_graph();
         for (void *p : allocs) cudaFree(p);
+        for (void *p : {(void *)read_jobs, (void *)read_w, (void *)read_stage}) cudaFree(p);
+        if (read_w_host) cudaFreeHost(read_w_host);
         if (rd_parts) cudaFreeHost(rd_parts);
         if (rd_perm) cudaFreeHost(rd_perm);
         if (side) cudaStreamDestroy(side);
@@ -414,6 +423,63 @@ int check_device_error(psf_batch *B)
     if (code != 0) return fail(PSF_ERR_TIMEOUT, "a tensor-core kernel gave up a bounded wait (code " +
                                                     std::to_string(code) + "); destroy the batch");
     return PSF_OK;
+}
+
+// Particles the staging buffer of grouped reads holds (64 MB), unless one slot
+// holds more.
+constexpr int64_t READ_STAGE = 4 << 20;
+
+// Buffers of a grouped read; false where memory for them is short.
+bool prepare_read(psf_batch *B, int64_t jobs, int64_t n_w, int64_t n_parts)
+{
+    auto grow = [B](void **p, int64_t *cap, int64_t need, size_t unit) {
+        if (need <= *cap) return true;
+        cudaFree(*p);
+        B->bytes -= *cap * (int64_t)unit;
+        *p = nullptr;
+        *cap = 0;
+        if (cudaMalloc(p, (size_t)need * unit) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        *cap = need;
+        B->bytes += need * (int64_t)unit;
+        return true;
+    };
+    if (n_w > B->read_host_cap) {
+        if (B->read_w_host) cudaFreeHost(B->read_w_host);
+        B->read_w_host = nullptr;
+        B->read_host_cap = 0;
+        if (cudaHostAlloc((void **)&B->read_w_host, (size_t)n_w * 8, cudaHostAllocDefault) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        B->read_host_cap = n_w;
+    }
+    const int64_t stage = std::min(n_parts, std::max(READ_STAGE, B->pmax_all));
+    return grow((void **)&B->read_w, &B->read_w_cap, n_w, sizeof(double)) &&
+           grow((void **)&B->read_jobs, &B->read_jobs_cap, jobs, sizeof(psf::ReadJob)) &&
+           grow((void **)&B->read_stage, &B->read_stage_cap, stage, sizeof(float4));
+}
+
+// The jobs of a read one after the other through the ordering scratch.
+int read_one_by_one(psf_batch *B, const std::vector<psf::ReadJob> &jobs, double *const *w, float *const *xyzw)
+{
+    for (size_t i = 0; i < jobs.size(); ++i) {
+        const psf::ReadJob &j = jobs[i];
+        if (j.n_w)
+            PSF_CUDA(cudaMemcpyAsync(w[i], j.w, (size_t)j.n_w * 8, cudaMemcpyDeviceToHost, B->stream));
+        if (j.n_parts) {
+            psf::PlainDev d{};
+            d.P = j.n_parts;
+            d.parts = B->pool_parts + j.poff;
+            d.perm = B->pool_perm + j.poff;
+            PSF_CHECK(psf::launch_unorder_particles(d, B->order, B->stream));
+            PSF_CUDA(cudaMemcpyAsync(xyzw[i], B->order.staging, (size_t)j.n_parts * 16, cudaMemcpyDeviceToHost,
+                                     B->stream));
+        }
+    }
+    return check_device_error(B);
 }
 
 int fused_grid(psf_batch *B)
@@ -906,27 +972,72 @@ int psf_batch_read_instances(psf_batch *B, int32_t n, const int32_t *basis, cons
 {
     if (!B || n < 0 || (n > 0 && (!basis || !slot || !w || !xyzw))) return fail(PSF_ERR_INVALID, "null argument");
     PSF_CUDA(cudaSetDevice(B->device));
+    std::vector<psf::ReadJob> jobs;
+    try {
+        jobs.resize((size_t)n);
+    } catch (const std::bad_alloc &) {
+        return fail(PSF_ERR_NOMEM, "host allocation failed");
+    }
+    int64_t n_w = 0, n_parts = 0;
     for (int32_t i = 0; i < n; ++i) {
         int sg = 0;
         PSF_CHECK(slot_index(B, basis[i], slot[i], &sg));
         const psf::SlotDev &s = B->slots[(size_t)sg];
         if (!s.active) return fail(PSF_ERR_STATE, "slot is empty");
-        HostGroup &G = B->groups[(size_t)basis[i]];
-        if (w[i])
-            PSF_CUDA(cudaMemcpyAsync(w[i], G.w + (size_t)slot[i] * G.N, (size_t)s.n_modes * 8, cudaMemcpyDeviceToHost,
-                                     B->stream));
-        if (xyzw[i] && s.n_particles > 0) {
-            // Scatter back to the caller's order in a per-slot region of the
-            // ordering scratch is not possible for several slots at once, so
-            // each slot is un-ordered into the staging buffer and copied.
-            PSF_CHECK(psf::launch_unorder_particles(particle_view(B, basis[i], slot[i], s.n_particles), B->order,
-                                                    B->stream));
-            PSF_CUDA(cudaMemcpyAsync(xyzw[i], B->order.staging, (size_t)s.n_particles * 16, cudaMemcpyDeviceToHost,
-                                     B->stream));
+        const HostGroup &G = B->groups[(size_t)basis[i]];
+        psf::ReadJob &j = jobs[(size_t)i];
+        j.w = G.w + (size_t)slot[i] * G.N;
+        j.poff = s.poff;
+        j.stage = 0;
+        j.n_w = w[i] ? s.n_modes : 0;
+        j.w_at = (int)n_w;
+        j.n_parts = xyzw[i] ? (int)s.n_particles : 0;
+        n_w += j.n_w;
+        n_parts += j.n_parts;
+    }
+    if (n < 2 || n > 65535 || !prepare_read(B, n, n_w, n_parts)) return read_one_by_one(B, jobs, w, xyzw);
+    // Groups of slots that fill the staging buffer: [first, last).
+    std::vector<std::pair<int32_t, int32_t>> groups;
+    for (int32_t i = 0; i < n;) {
+        const int32_t first = i;
+        int64_t at = 0;
+        for (; i < n && at + jobs[(size_t)i].n_parts <= B->read_stage_cap; ++i) {
+            jobs[(size_t)i].stage = at;
+            at += jobs[(size_t)i].n_parts;
+        }
+        groups.emplace_back(first, i);
+    }
+    cudaStream_t st = B->stream;
+    PSF_CUDA(cudaMemcpyAsync(B->read_jobs, jobs.data(), jobs.size() * sizeof(psf::ReadJob), cudaMemcpyHostToDevice, st));
+    if (n_w > 0) {
+        PSF_CHECK(psf::launch_batch_gather_states(B->read_jobs, n, B->read_w, st));
+        PSF_CUDA(cudaMemcpyAsync(B->read_w_host, B->read_w, (size_t)n_w * 8, cudaMemcpyDeviceToHost, st));
+    }
+    for (const auto &g : groups) {
+        int most = 0;
+        for (int32_t i = g.first; i < g.second; ++i) most = std::max(most, jobs[(size_t)i].n_parts);
+        if (most == 0) continue;
+        PSF_CHECK(psf::launch_batch_unorder(B->read_jobs + g.first, g.second - g.first, most, B->pool_parts,
+                                            B->pool_perm, B->read_stage, st));
+        // One copy for slots whose host buffers follow one another.
+        for (int32_t i = g.first; i < g.second;) {
+            const int32_t first = i;
+            int64_t count = 0;
+            do {
+                count += jobs[(size_t)i].n_parts;
+                ++i;
+            } while (i < g.second && (jobs[(size_t)i].n_parts == 0 || xyzw[i] == xyzw[first] + 4 * count) &&
+                     jobs[(size_t)first].n_parts > 0);
+            if (count > 0)
+                PSF_CUDA(cudaMemcpyAsync(xyzw[first], B->read_stage + jobs[(size_t)first].stage, (size_t)count * 16,
+                                         cudaMemcpyDeviceToHost, st));
         }
     }
-    PSF_CUDA(cudaStreamSynchronize(B->stream));
-    return check_device_error(B);
+    PSF_CHECK(check_device_error(B));
+    for (int32_t i = 0; i < n; ++i)
+        if (jobs[(size_t)i].n_w)
+            std::memcpy(w[i], B->read_w_host + jobs[(size_t)i].w_at, (size_t)jobs[(size_t)i].n_w * 8);
+    return PSF_OK;
 }
 
 int psf_batch_pool_free(psf_batch *B, int64_t *free_particles, int64_t *largest_range)

@@ -118,6 +118,20 @@ int launch_batch_state(const GroupDev *groups, SlotDev *slots, int n_slots, cuda
 // prefix[s] = particles of slots 0..s-1 (occupied slots only); n_slots + 1 entries.
 int launch_batch_trace(const GroupDev *groups, const SlotDev *slots, const long long *prefix, int n_slots, int grid,
                        bool all_centred, bool faces, cudaStream_t st, bool after_kernel = false);
+// One slot of a grouped read-back: its state row, its particles in the pool and
+// where both go in the staging buffers.
+struct ReadJob {
+    const double *w;
+    long long poff, stage;  // first particle in the pool and in the staging buffer
+    int n_w, w_at;          // state values (0: not wanted) and their place
+    int n_parts;            // particles in this group of jobs (0: none)
+};
+
+// Gather the jobs' states into `w_out`, and their particles, in the caller's
+// order, into `stage`.
+int launch_batch_gather_states(const ReadJob *jobs, int n, double *w_out, cudaStream_t st);
+int launch_batch_unorder(const ReadJob *jobs, int n, int max_parts, const float4 *pool, const int32_t *perm,
+                         float4 *stage, cudaStream_t st);
 int launch_batch_pack(const GroupDev *groups, const SlotDev *slots, int slot_global, cudaStream_t st);
 int batch_trace_grid(int num_sms, bool faces);
 
