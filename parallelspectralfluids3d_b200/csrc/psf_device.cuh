@@ -1,6 +1,6 @@
 // Device helpers shared by the single-instance and the batched kernels:
 // reference face numbering, the staggered trilinear interpolant, one
-// particle step, the respawn generator, Morton keys and FP64 reductions.
+// particle step, the respawn generator and FP64 reductions.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -434,19 +434,6 @@ __device__ __forceinline__ float4 advance_particle(float4 p, const GridDev &g, P
         p.w = (float)((double)tp.lifetime * ((double)r2 / 1024.0));
     }
     return p;
-}
-
-// ------------------------------------------------------- particle order
-// Particles are kept sorted by the Morton code of their voxel so that the
-// threads of a warp gather from a few neighbouring cells of the face field.
-__device__ __forceinline__ uint32_t spread10(uint32_t v)
-{
-    v &= 0x3ffu;
-    v = (v | (v << 16)) & 0x030000FFu;
-    v = (v | (v << 8)) & 0x0300F00Fu;
-    v = (v | (v << 4)) & 0x030C30C3u;
-    v = (v | (v << 2)) & 0x09249249u;
-    return v;
 }
 
 }  // namespace psf

@@ -62,7 +62,7 @@ struct PlainDev {
     const unsigned long long *trace_ctr;      // step count of the state the tracer advects with
     const int32_t *pair_dst;  // [n_active][2] float indices into pairs of each active face
     int trace_blocks;    // persistent tracer grid: SMs x resident blocks per SM
-    float4 *parts;       // [P] in cell (Morton) order
+    float4 *parts;       // [P] in brick order (psf_particle_keys)
     const int32_t *perm; // [P] caller index of each stored particle
     GridDev grid;
     StateParams sp;
@@ -112,7 +112,7 @@ int launch_reconstruct(const PlainDev &d, cudaStream_t st, bool after_kernel = t
 int launch_trace(const PlainDev &d, cudaStream_t st, bool after_kernel = true);
 int trace_blocks_per_sm();
 int sort_particles_temp_bytes(long long P, size_t *bytes);
-// Put caller-order particles (o.staging) into cell order: a Morton sort that
+// Put caller-order particles (o.staging) into brick order: a sort that
 // rewrites d.perm, or with `resort` false a gather through the current perm.
 int launch_order_particles(const PlainDev &d, const OrderBufs &o, cudaStream_t st, bool resort = true);
 int launch_unorder_particles(const PlainDev &d, const OrderBufs &o, cudaStream_t st);
