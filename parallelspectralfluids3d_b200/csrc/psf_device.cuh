@@ -292,16 +292,16 @@ struct Trilinear {
 // the unclamped origin.
 //
 // Bound by the latency and L1 lookups of the gathers (RK1, which has one per
-// particle and little else, takes 80 us where RK4 takes 102).  Against three
-// cell keys and nested lerps, 16 x 262,144 particles on the 32^3 box with a
-// sphere, RK4: 102 against 111 us at 0.001 voxel per step, 129 against 133 us
-// at 0.03; 513 x 16,384 on three domains: 284 against 297 us.  Storing the
-// pairs in bricks of 4 x 2 x 2 voxels made RK1 73 us but RK4 139 us (the
-// places cost more in the repeated gathers) and the 512-slot reconstruction
-// 353 against 302 us; storing every face once (24 loads of 4 bytes) was slower
-// at every density.
+// particle and little else, takes 70 us where RK4 takes 96 on 16 x 262,144
+// particles of the 32^3 box with a sphere).  Measured with particles in Morton
+// order, against three cell keys and nested lerps: 102 against 111 us at 0.001
+// voxel per step, 129 against 133 us at 0.03; 513 x 16,384 on three domains: 284
+// against 297 us.  Storing the pairs in bricks of 4 x 2 x 2 voxels made RK1 73
+// instead of 80 us but RK4 139 instead of 129 (the places cost more in the
+// repeated gathers) and the 512-slot reconstruction 353 instead of 302.
 template <class Field>
 struct CentredBox {
+    using Ptr = typename Field::Ptr;
     float ox, oy, oz;     // whole-cell origin
     float sx, sy, sz;     // half-shifted origin
     Trilinear x, y, z;
@@ -346,6 +346,17 @@ struct CentredBox {
         return __float_as_uint(fminf(a, b)) <= 0x3F000000u;  // [0, 1/2]
     }
 
+    // Velocity at a position that lies in the gathered half-cell; false where it
+    // does not.
+    __device__ __forceinline__ bool velocity_inside(const GridDev &g, float px, float py, float pz, float3 &v) const
+    {
+        const float qx = px - g.mn[0], qy = py - g.mn[1], qz = pz - g.mn[2];
+        const float ax = fmaf(qx, g.inv_h, -ox), ay = fmaf(qy, g.inv_h, -oy), az = fmaf(qz, g.inv_h, -oz);
+        const float bx = fmaf(qx, g.inv_h, -sx), by = fmaf(qy, g.inv_h, -sy), bz = fmaf(qz, g.inv_h, -sz);
+        v = make_float3(x.at(ax, by, bz), y.at(bx, ay, bz), z.at(bx, by, az));
+        return inside(ax, bx) && inside(ay, by) && inside(az, bz);
+    }
+
     __device__ __forceinline__ float3 velocity(const GridDev &g, typename Field::Ptr u, float px, float py, float pz)
     {
         const float qx = px - g.mn[0], qy = py - g.mn[1], qz = pz - g.mn[2];
@@ -379,6 +390,42 @@ __device__ __forceinline__ float div6(float x)
     const float r = 1.0f / 6.0f;
     const float q = x * r;
     return fmaf(fmaf(-q, 6.0f, x), r, q);
+}
+
+// A particle's step whose stages all stay in its first half-cell: the same
+// operations as advance_particle, with one gather and no other path.  False
+// (and p as it was) where a stage leaves it or the particle's life is over.
+template <class Field>
+__device__ __forceinline__ bool advance_inside(float4 &p, const GridDev &g, typename Field::Ptr u,
+                                               const TraceParams &tp)
+{
+    if (!(p.w > 0.f)) return false;
+    const float dt = tp.dt;
+    CentredBox<Field> box;
+    float3 v = box.velocity(g, u, p.x, p.y, p.z);
+    bool stays = true;
+    if (tp.rk4) {
+        const float3 k1 = v;
+        float3 k2, k3, k4;
+        stays = box.velocity_inside(g, clampf(p.x + 0.5f * dt * k1.x, g.mn[0], g.mx[0]),
+                                    clampf(p.y + 0.5f * dt * k1.y, g.mn[1], g.mx[1]),
+                                    clampf(p.z + 0.5f * dt * k1.z, g.mn[2], g.mx[2]), k2);
+        stays &= box.velocity_inside(g, clampf(p.x + 0.5f * dt * k2.x, g.mn[0], g.mx[0]),
+                                     clampf(p.y + 0.5f * dt * k2.y, g.mn[1], g.mx[1]),
+                                     clampf(p.z + 0.5f * dt * k2.z, g.mn[2], g.mx[2]), k3);
+        stays &= box.velocity_inside(g, clampf(p.x + dt * k3.x, g.mn[0], g.mx[0]),
+                                     clampf(p.y + dt * k3.y, g.mn[1], g.mx[1]),
+                                     clampf(p.z + dt * k3.z, g.mn[2], g.mx[2]), k4);
+        v.x = div6(k1.x + 2.f * k2.x + 2.f * k3.x + k4.x);
+        v.y = div6(k1.y + 2.f * k2.y + 2.f * k3.y + k4.y);
+        v.z = div6(k1.z + 2.f * k2.z + 2.f * k3.z + k4.z);
+    }
+    if (!stays) return false;
+    p.x = clampf(p.x + dt * v.x, g.mn[0], g.mx[0]);
+    p.y = clampf(p.y + dt * v.y, g.mn[1], g.mx[1]);
+    p.z = clampf(p.z + dt * v.z, g.mn[2], g.mx[2]);
+    p.w = p.w - 1.f;
+    return true;
 }
 
 // One particle step (psfsolver.cpp:75-224): RK1 or RK4 with the box clamp
