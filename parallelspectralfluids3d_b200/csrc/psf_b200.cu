@@ -305,45 +305,12 @@ __global__ void __launch_bounds__(TRACE_THREADS, 3) psf_trace(float4 *__restrict
     }
 }
 
-// Storage order of particles: bricks of 16 x 2 x 2 voxels, in a brick the
-// half-cells' rows along x.  A face field's rows run along x too, so the lanes
-// of a warp gather from few 128-byte lines (a Morton order's 32 particles lie
-// in twice as many rows), while a block's particles still share the rows in its
-// L1.  Against Morton order: 64 x 16,384 particles on 64 x 32 x 32 41 against 51
-// us, 513 x 16,384 on three domains 268 against 321 us, 16 x 262,144 on 32^3 RK1
-// 70 against 80 us, RK4 99 against 102 us.
-constexpr int BRICK_X = 4, BRICK_Y = 1, BRICK_Z = 1;                   // log2 of a brick's voxels
-constexpr int BRICK_BITS = BRICK_X + (BRICK_Y + 1) + (BRICK_Z + 1);  // of a key, below the brick's number
-
-struct Bricks {
-    uint32_t nx, ny, nz;
-    int key_bits;
-};
-
-// At 1023 voxels per axis 64 x 512 x 512 bricks: 24 + 8 bits.
-Bricks bricks_of(const GridDev &g)
-{
-    Bricks b;
-    b.nx = ((uint32_t)g.nx + (1u << BRICK_X) - 1) >> BRICK_X;
-    b.ny = ((uint32_t)g.ny + (1u << BRICK_Y) - 1) >> BRICK_Y;
-    b.nz = ((uint32_t)g.nz + (1u << BRICK_Z) - 1) >> BRICK_Z;
-    b.key_bits = BRICK_BITS;
-    while (((uint64_t)1 << (b.key_bits - BRICK_BITS)) < (uint64_t)b.nx * b.ny * b.nz) ++b.key_bits;
-    return b;
-}
-
 __global__ void psf_particle_keys(const float4 *__restrict__ in, long long P, GridDev g, Bricks b,
                                   uint32_t *__restrict__ keys, int32_t *__restrict__ idx)
 {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P) return;
-    const float4 p = in[i];
-    const uint32_t x = (uint32_t)clampi(__float2int_rd((p.x - g.mn[0]) * g.inv_h), 0, g.nx - 1);
-    const uint32_t hy = (uint32_t)clampi(__float2int_rd(2.0f * ((p.y - g.mn[1]) * g.inv_h)), 0, 2 * g.ny - 1);
-    const uint32_t hz = (uint32_t)clampi(__float2int_rd(2.0f * ((p.z - g.mn[2]) * g.inv_h)), 0, 2 * g.nz - 1);
-    const uint32_t brick = ((hz >> (BRICK_Z + 1)) * b.ny + (hy >> (BRICK_Y + 1))) * b.nx + (x >> BRICK_X);
-    const uint32_t row = ((hz & ((2u << BRICK_Z) - 1)) << (BRICK_Y + 1)) | (hy & ((2u << BRICK_Y) - 1));
-    keys[i] = (brick << BRICK_BITS) | (row << BRICK_X) | (x & ((1u << BRICK_X) - 1));
+    keys[i] = b.key(g, in[i]);
     idx[i] = (int32_t)i;
 }
 

@@ -153,6 +153,8 @@ struct psf_batch {
     float4 *pool_parts = nullptr;   // particle pool shared by all slots
     int32_t *pool_perm = nullptr;
     int64_t pool_cap = 0;           // particles
+    int since_order = 0;            // steps since the last launch_batch_reorder
+    int order_round = 0;
     RangePool pool;
     std::vector<int64_t> slot_units;  // pool units held by each slot
     int64_t bytes = 0;
@@ -602,6 +604,9 @@ int launch_step(psf_batch *B, cudaStream_t st, bool after_kernel)
 // 184 us).  Nor the state update, whose blocks hold up the contraction's end
 // (67.5 us for 40 of N = 200).
 constexpr int RUN_STEPS = 8;
+
+// Steps between two looks at the particles' order (psf_batch_reorder).
+constexpr int ORDER_EVERY = 64;
 
 int build_graph(psf_batch *B, int which)
 {
@@ -1057,7 +1062,15 @@ int psf_batch_step(psf_batch *B, int32_t nsteps)
         const int which = nsteps >= RUN_STEPS ? 1 : 0;
         PSF_CHECK(build_graph(B, which));
         PSF_CUDA(cudaGraphLaunch(B->execs[which], B->stream));
-        nsteps -= which ? RUN_STEPS : 1;
+        const int taken = which ? RUN_STEPS : 1;
+        nsteps -= taken;
+        B->since_order += taken;
+        if (B->since_order >= ORDER_EVERY && B->prefix.back() > 0) {
+            B->since_order = 0;
+            B->order_round = B->order_round == INT32_MAX ? 1 : B->order_round + 1;
+            PSF_CHECK(psf::launch_batch_reorder(B->d_groups, B->d_slots, B->d_prefix, B->n_slots(), B->prefix.back(),
+                                                B->order_round, B->stream));
+        }
     }
     return PSF_OK;
 }

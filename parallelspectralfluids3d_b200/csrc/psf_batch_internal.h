@@ -84,7 +84,7 @@ struct SlotDev {
     long long poff;           // first particle of the slot in the particle pool
     unsigned long long target;  // stop after this many steps (0: no limit)
     int stepped;              // 1 if the slot advanced in the current step (set by the state kernel)
-    int pad1;
+    int mixed;                // round of launch_batch_reorder in which the slot was out of order
 };
 
 // Per-basis device view used by the state kernel and the tracer.
@@ -118,6 +118,10 @@ int launch_batch_state(const GroupDev *groups, SlotDev *slots, int n_slots, cuda
 // prefix[s] = particles of slots 0..s-1 (occupied slots only); n_slots + 1 entries.
 int launch_batch_trace(const GroupDev *groups, const SlotDev *slots, const long long *prefix, int n_slots, int grid,
                        bool all_centred, bool faces, cudaStream_t st, bool after_kernel = false);
+// Put the particles of slots that go on stepping back in brick order where the
+// flow has mixed them.  `round` differs from call to call; `total` is prefix[n_slots].
+int launch_batch_reorder(const GroupDev *groups, SlotDev *slots, const long long *prefix, int n_slots, long long total,
+                         int round, cudaStream_t st);
 // One slot of a grouped read-back: its state row, its particles in the pool and
 // where both go in the staging buffers.
 struct ReadJob {
