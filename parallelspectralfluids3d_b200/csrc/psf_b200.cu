@@ -2,7 +2,8 @@
 // include/psf_b200.h for single-instance contexts.
 //
 // One step (the reference's PSFSolver::integrate, Solver/SolverImpl/
-// psfsolver.cpp:21-234) is three kernels, captured once into a CUDA graph:
+// psfsolver.cpp:21-234) is three kernels, replayed from CUDA graphs of one step
+// or a run of steps:
 //
 //   1. psf_contract_state  dw_k = sum_a w_a sum_j C[k][a][j] w_j over an FP32
 //      C streamed with 128-bit loads, FP64 accumulation; the last CTA to
@@ -281,10 +282,11 @@ __global__ void __launch_bounds__(256) psf_reconstruct(const float *__restrict__
 }
 
 // Persistent grid (a whole number of resident blocks per SM) striding over
-// the particles, which are stored in cell order.  A thread's first particle
+// the particles, which are stored in brick order.  A thread's first particle
 // is loaded before the grid-dependency wait: the particles were last written
-// by the previous step's tracer, which belongs to an earlier graph launch
-// (or an earlier, synchronised profiling step).
+// by the previous step's tracer, which belongs to an earlier graph launch or,
+// in a run, has ended when this one starts (or to an earlier, synchronised
+// profiling step).
 constexpr int TRACE_THREADS = 256;
 
 template <class Box>
