@@ -164,6 +164,11 @@ using psf::n_faces_of;
 // have buffers of their own.
 constexpr int RUN_STEPS = 12;
 constexpr int RUN_EXTRA = RUN_STEPS - 3;
+// A run's graph is captured once this many steps that could have gone into runs
+// were taken one by one.  Capturing and loading it takes 0.95 ms and a step in a
+// run is 2.2 to 6 us shorter, so about this many steps pay for it; a context
+// closed earlier pays nothing, and the latest to gain loses 1 ms once.
+constexpr int RUN_AFTER = 288;
 
 struct psf_ctx {
     int device = 0;
@@ -176,6 +181,7 @@ struct psf_ctx {
     cudaGraphExec_t execs[3][6] = {};
     cudaGraph_t run_graphs[6] = {};             // RUN_STEPS steady steps, by the position they start from
     cudaGraphExec_t run_execs[6] = {};
+    int singles = 0;                            // steps taken singly, since the last capture, that a run could have held
     double *wbuf[3 + RUN_EXTRA] = {};           // the ring, then the states between a run's first and last three
     unsigned long long *ctrbuf = nullptr;       // completed steps of each slot's state
     float *ubuf[2] = {nullptr, nullptr};
@@ -229,6 +235,7 @@ struct psf_ctx {
             run_execs[i] = nullptr;
             run_graphs[i] = nullptr;
         }
+        singles = 0;
     }
     int slot(int k) const { return (vis + k) % 3; }
     static int slot_of(int v, int k) { return (v + k) % 3; }
@@ -392,7 +399,7 @@ static int capture_step(psf_ctx *c, int kind, int v, int q, cudaGraph_t *out)
 // 262,144 particles 17.2 against 20.4; 48^3, N = 256, 1 M particles 75 against
 // 81.  What is left is the reconstruction and the tracer, each of which fills
 // the chip by itself.  RUN_STEPS = 12 keeps a rollout of 50 steps mostly in
-// runs and the capture below 0.2 ms.
+// runs.
 static int capture_run(psf_ctx *c, int v, int q, cudaGraph_t *out)
 {
     cudaStream_t m = c->stream, s0 = c->side[0], s1 = c->side[1];
@@ -439,22 +446,25 @@ static int capture_run(psf_ctx *c, int v, int q, cudaGraph_t *out)
     return PSF_OK;
 }
 
-// Launch RUN_STEPS steps of a primed pipeline.
-static int launch_run(psf_ctx *c)
+// Whether RUN_STEPS steps of a primed pipeline can go in one launch from the
+// current ring position.  Where they cannot, single steps soon reach a position
+// that has its graph, as the six positions follow one another.
+static int ready_run(psf_ctx *c, bool *ready)
 {
     const int idx = c->vis * 2 + c->tq;
-    if (!c->run_execs[idx]) {
+    if (!c->run_execs[idx] && c->singles >= RUN_AFTER) {
         cudaGraph_t g = nullptr;
         PSF_CHECK(capture_run(c, c->vis, c->tq, &g));
         c->run_graphs[idx] = g;
         PSF_CUDA(cudaGraphInstantiate(&c->run_execs[idx], g, 0));
+        c->singles = 0;
     }
-    PSF_CUDA(cudaGraphLaunch(c->run_execs[idx], c->stream));
+    *ready = c->run_execs[idx] != nullptr;
     return PSF_OK;
 }
 
-// Launch one step and rotate the ring.  A position of a step kind is captured
-// the first time it is needed.
+// Launch one step and rotate the ring.  A kind's six ring positions are captured
+// together the first time it is needed.
 static int launch_step(psf_ctx *c)
 {
     const int kind = c->primed ? STEP_STEADY : (c->changed ? STEP_LEAN : STEP_BOOT);
@@ -471,10 +481,15 @@ static int launch_step(psf_ctx *c)
         return PSF_OK;
     }
     if (!c->execs[kind][idx]) {
-        cudaGraph_t g = nullptr;
-        PSF_CHECK(capture_step(c, kind, c->vis, c->tq, &g));
-        c->graphs[kind][idx] = g;
-        PSF_CUDA(cudaGraphInstantiate(&c->execs[kind][idx], g, 0));
+        for (int v = 0; v < 3; ++v)
+            for (int q = 0; q < 2; ++q) {
+                const int i = v * 2 + q;
+                if (c->execs[kind][i]) continue;
+                cudaGraph_t g = nullptr;
+                PSF_CHECK(capture_step(c, kind, v, q, &g));
+                c->graphs[kind][i] = g;
+                PSF_CUDA(cudaGraphInstantiate(&c->execs[kind][i], g, 0));
+            }
     }
     PSF_CUDA(cudaGraphLaunch(c->execs[kind][idx], c->stream));
     c->vis = c->slot(1);
@@ -797,8 +812,15 @@ int psf_step(psf_ctx *c, int32_t nsteps)
     if (!c->have_state) return fail(PSF_ERR_STATE, "psf_set_state must be called before stepping");
     PSF_CUDA(cudaSetDevice(c->device));
     while (nsteps > 0) {
-        const bool run = c->primed && nsteps >= RUN_STEPS;
-        PSF_CHECK(run ? launch_run(c) : launch_step(c));
+        bool run = false;
+        if (c->primed && nsteps >= RUN_STEPS) {
+            PSF_CHECK(ready_run(c, &run));
+            if (!run) ++c->singles;
+        }
+        if (run)
+            PSF_CUDA(cudaGraphLaunch(c->run_execs[c->vis * 2 + c->tq], c->stream));
+        else
+            PSF_CHECK(launch_step(c));
         nsteps -= run ? RUN_STEPS : 1;
     }
     return PSF_OK;

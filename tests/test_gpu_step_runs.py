@@ -1,4 +1,7 @@
-"""Runs of steady steps in one graph: any split of a rollout gives the same bits as single steps."""
+"""Runs of steady steps in one graph: any split of a rollout gives the same bits as single steps.
+
+Runs begin once 288 steps were taken singly.
+"""
 import numpy as np
 import pytest
 
@@ -29,7 +32,7 @@ def outcome(b, splits, particles):
 
 
 @pytest.mark.parametrize("particles", [True, False])
-@pytest.mark.parametrize("counts", [(14, 12, 11), (13, 25, 1, 24), (2, 36, 5, 17), (40,)])
+@pytest.mark.parametrize("counts", [(314, 12, 11), (113, 225, 1, 24), (2, 336, 5, 17, 290, 330), (40, 400)])
 def test_runs_equal_single_steps(small_bases, particles, counts):
     b = small_bases["sphere12x10x9"]
     whole = outcome(b, [[n] for n in counts], particles)
@@ -43,10 +46,10 @@ def test_runs_after_changes(small_bases):
     """A change of state between runs restarts the pipeline; parameters drop the captured graphs."""
     b = small_bases["box576"]
     got = []
-    for split in ([30, 16, 28], None):
+    for split in ([330, 16, 360], None):
         with Context(b, L.make_params(dt=0.01)) as ctx:
             ctx.set_particles(initial_particles(b, 500, 2))
-            for k, n in enumerate([30, 16, 28]):
+            for k, n in enumerate([330, 16, 360]):
                 if k == 2:
                     ctx.set_params(L.make_params(dt=0.02, integrator=L.PSF_RK1))
                 else:
