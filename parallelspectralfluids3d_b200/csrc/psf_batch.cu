@@ -1082,16 +1082,25 @@ void split_bf16_host(double x, uint16_t *hi, uint16_t *lo)
     std::memcpy(lo, &l, 2);
 }
 
+int prepare_batch_reorder()
+{
+    for (int deal = 0; deal < 2; ++deal) {
+        auto kernel = deal ? psf_batch_reorder<true> : psf_batch_reorder<false>;
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ORDER_SMEM);
+        if (e != cudaSuccess) return cuda_fail(e, "psf_batch_reorder shared memory");
+    }
+    return PSF_OK;
+}
+
 int launch_batch_reorder(const GroupDev *groups, SlotDev *slots, const long long *prefix, int n_slots, long long total,
                          int round, cudaStream_t st)
 {
     const long long blocks = total / ORDER_WINDOW + n_slots;
     for (int deal = 0; deal < 2; ++deal) {
         auto kernel = deal ? psf_batch_reorder<true> : psf_batch_reorder<false>;
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ORDER_SMEM);
-        if (e != cudaSuccess) return cuda_fail(e, "psf_batch_reorder shared memory");
         kernel<<<(unsigned)blocks, ORDER_BLOCK, ORDER_SMEM, st>>>(groups, slots, prefix, n_slots, round);
-        if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "psf_batch_reorder launch");
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return cuda_fail(e, "psf_batch_reorder launch");
     }
     return PSF_OK;
 }

@@ -787,6 +787,7 @@ int psf_batch_create(const psf_batch_config *cfg, int device, psf_batch **out)
     fill_gemm_args(B);
     if ((rc = upload_tables(B)) != PSF_OK || (rc = upload_prefix(B)) != PSF_OK) return bail(rc);
     B->trace_ctas = psf::batch_trace_grid(B->num_sms, B->face_field);
+    if ((rc = psf::prepare_batch_reorder()) != PSF_OK) return bail(rc);
     B->gemm_ctas = cfg->gemm_ctas > 0 ? cfg->gemm_ctas : B->num_sms;
     if (cfg->gemm_columns != 0) {
         B->bn_max = cfg->gemm_columns;

@@ -120,6 +120,8 @@ int launch_batch_trace(const GroupDev *groups, const SlotDev *slots, const long 
                        bool all_centred, bool faces, cudaStream_t st, bool after_kernel = false);
 // Put the particles of slots that go on stepping back in brick order where the
 // flow has mixed them.  `round` differs from call to call; `total` is prefix[n_slots].
+// prepare_batch_reorder loads the kernels on the current device, so that no step waits for it.
+int prepare_batch_reorder();
 int launch_batch_reorder(const GroupDev *groups, SlotDev *slots, const long long *prefix, int n_slots, long long total,
                          int round, cudaStream_t st);
 // One slot of a grouped read-back: its state row, its particles in the pool and
