@@ -464,6 +464,47 @@ bool prepare_read(psf_batch *B, int64_t jobs, int64_t n_w, int64_t n_parts)
            grow((void **)&B->read_stage, &B->read_stage_cap, stage, sizeof(float4));
 }
 
+// Where the host memory that one copy may cover ends, starting from a host
+// pointer.  Buffers that follow one another need not be one allocation, and a
+// copy over memory that is registered in part, or by two registrations, is
+// refused; so a copy is not taken past the allocation it starts in.
+struct CopyRange {
+    enum { ALONE, PAGEABLE, REGISTERED } kind = ALONE;
+    uintptr_t end = 0;  // of the registered allocation
+
+    explicit CopyRange(const void *p)
+    {
+        cudaPointerAttributes a{};
+        if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+            cudaGetLastError();
+            return;
+        }
+        if (a.type == cudaMemoryTypeUnregistered) kind = PAGEABLE;
+        if (a.type != cudaMemoryTypeHost) return;
+        void *fn = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuPointerGetAttribute", &fn, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess || !fn) {
+            cudaGetLastError();
+            return;
+        }
+        auto get = reinterpret_cast<decltype(&cuPointerGetAttribute)>(fn);
+        CUdeviceptr start = 0;
+        size_t size = 0;
+        if (get(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, (CUdeviceptr)(uintptr_t)p) != CUDA_SUCCESS ||
+            get(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, (CUdeviceptr)(uintptr_t)p) != CUDA_SUCCESS)
+            return;
+        kind = REGISTERED;
+        end = (uintptr_t)start + size;
+    }
+    // Whether the buffer at p, which follows what is covered so far, is covered too.
+    bool covers(const void *p, size_t bytes) const
+    {
+        if (kind == REGISTERED) return (uintptr_t)p + bytes <= end;
+        return kind == PAGEABLE && CopyRange(p).kind == PAGEABLE;
+    }
+};
+
 // The jobs of a read one after the other through the ordering scratch.
 int read_one_by_one(psf_batch *B, const std::vector<psf::ReadJob> &jobs, double *const *w, float *const *xyzw)
 {
@@ -1004,14 +1045,18 @@ int psf_batch_read_instances(psf_batch *B, int32_t n, const int32_t *basis, cons
     if (n < 2 || n > 65535 || !prepare_read(B, n, n_w, n_parts)) return read_one_by_one(B, jobs, w, xyzw);
     // Groups of slots that fill the staging buffer: [first, last).
     std::vector<std::pair<int32_t, int32_t>> groups;
-    for (int32_t i = 0; i < n;) {
-        const int32_t first = i;
-        int64_t at = 0;
-        for (; i < n && at + jobs[(size_t)i].n_parts <= B->read_stage_cap; ++i) {
-            jobs[(size_t)i].stage = at;
-            at += jobs[(size_t)i].n_parts;
+    try {
+        for (int32_t i = 0; i < n;) {
+            const int32_t first = i;
+            int64_t at = 0;
+            for (; i < n && at + jobs[(size_t)i].n_parts <= B->read_stage_cap; ++i) {
+                jobs[(size_t)i].stage = at;
+                at += jobs[(size_t)i].n_parts;
+            }
+            groups.emplace_back(first, i);
         }
-        groups.emplace_back(first, i);
+    } catch (const std::bad_alloc &) {
+        return fail(PSF_ERR_NOMEM, "host allocation failed");
     }
     cudaStream_t st = B->stream;
     PSF_CUDA(cudaMemcpyAsync(B->read_jobs, jobs.data(), jobs.size() * sizeof(psf::ReadJob), cudaMemcpyHostToDevice, st));
@@ -1025,18 +1070,24 @@ int psf_batch_read_instances(psf_batch *B, int32_t n, const int32_t *basis, cons
         if (most == 0) continue;
         PSF_CHECK(psf::launch_batch_unorder(B->read_jobs + g.first, g.second - g.first, most, B->pool_parts,
                                             B->pool_perm, B->read_stage, st));
-        // One copy for slots whose host buffers follow one another.
+        // One copy for slots whose host buffers follow one another in one piece of memory.
         for (int32_t i = g.first; i < g.second;) {
             const int32_t first = i;
-            int64_t count = 0;
-            do {
-                count += jobs[(size_t)i].n_parts;
-                ++i;
-            } while (i < g.second && (jobs[(size_t)i].n_parts == 0 || xyzw[i] == xyzw[first] + 4 * count) &&
-                     jobs[(size_t)first].n_parts > 0);
-            if (count > 0)
-                PSF_CUDA(cudaMemcpyAsync(xyzw[first], B->read_stage + jobs[(size_t)first].stage, (size_t)count * 16,
-                                         cudaMemcpyDeviceToHost, st));
+            const auto follows = [&](int32_t k, int64_t count) { return xyzw[k] == xyzw[first] + 4 * count; };
+            int64_t count = jobs[(size_t)i++].n_parts;
+            if (count == 0) continue;
+            while (i < g.second && jobs[(size_t)i].n_parts == 0) ++i;
+            if (i < g.second && follows(i, count)) {
+                const CopyRange range(xyzw[first]);
+                while (i < g.second && (jobs[(size_t)i].n_parts == 0 ||
+                                        (follows(i, count) &&
+                                         range.covers(xyzw[i], (size_t)jobs[(size_t)i].n_parts * 16)))) {
+                    count += jobs[(size_t)i].n_parts;
+                    ++i;
+                }
+            }
+            PSF_CUDA(cudaMemcpyAsync(xyzw[first], B->read_stage + jobs[(size_t)first].stage, (size_t)count * 16,
+                                     cudaMemcpyDeviceToHost, st));
         }
     }
     PSF_CHECK(check_device_error(B));
