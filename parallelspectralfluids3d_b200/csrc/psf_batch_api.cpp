@@ -159,12 +159,15 @@ struct psf_batch {
     std::vector<int64_t> slot_units;  // pool units held by each slot
     int64_t bytes = 0;
     std::vector<void *> allocs;
-    // Grouped reads (psf_batch_read_instances): job table, gathered states with
-    // a pinned copy, and staging for READ_STAGE particles (or the largest slot).
-    psf::ReadJob *read_jobs = nullptr;
-    double *read_w = nullptr, *read_w_host = nullptr;
-    int64_t read_jobs_cap = 0, read_w_cap = 0, read_host_cap = 0, read_stage_cap = 0;
+    // Grouped reads (psf_batch_read_instances): staging for READ_STAGE particles
+    // (or the largest slot), gathered states with a pinned copy, and job table, in
+    // one allocation that read_stage begins.
     float4 *read_stage = nullptr;
+    double *read_w = nullptr, *read_w_host = nullptr;
+    psf::ReadJob *read_jobs = nullptr;
+    int64_t read_w_cap = 0, read_stage_cap = 0;
+    int64_t read_slots = 0;      // slots asked for before the buffers were made
+    bool reads_singly = false;   // no memory for them
     // Reads of slots that the queued steps do not touch (psf::batch_read_frozen):
     // a second stream and pinned host buffers for one slot's particles.
     cudaStream_t side = nullptr;
@@ -178,7 +181,7 @@ struct psf_batch {
     {
         drop_graph();
         for (void *p : allocs) cudaFree(p);
-        for (void *p : {(void *)read_jobs, (void *)read_w, (void *)read_stage}) cudaFree(p);
+        cudaFree(read_stage);
         if (read_w_host) cudaFreeHost(read_w_host);
         if (rd_parts) cudaFreeHost(rd_parts);
         if (rd_perm) cudaFreeHost(rd_perm);
@@ -430,38 +433,44 @@ int check_device_error(psf_batch *B)
 // Particles the staging buffer of grouped reads holds (64 MB), unless one slot
 // holds more.
 constexpr int64_t READ_STAGE = 4 << 20;
+// Their buffers are made once, for the largest read, by the read with which so
+// many slots have been asked for: 0.5 to 2 ms, and a grouped read is 9 to 16 us a
+// slot shorter (two slots 53 -> 44 us, 64 slots of 4,096 particles 890 -> 124,
+// 96 of 65,536 3.48 -> 1.88 ms).  A batch that is read less than that pays nothing.
+constexpr int64_t READ_AFTER = 128;
 
-// Buffers of a grouped read; false where memory for them is short.
-bool prepare_read(psf_batch *B, int64_t jobs, int64_t n_w, int64_t n_parts)
+// Whether a read of n slots goes through the buffers of grouped reads; not where
+// memory for them is short.
+bool group_read(psf_batch *B, int64_t n, int64_t n_w)
 {
-    auto grow = [B](void **p, int64_t *cap, int64_t need, size_t unit) {
-        if (need <= *cap) return true;
-        cudaFree(*p);
-        B->bytes -= *cap * (int64_t)unit;
-        *p = nullptr;
-        *cap = 0;
-        if (cudaMalloc(p, (size_t)need * unit) != cudaSuccess) {
+    const int64_t jobs = B->n_slots();
+    if (n < 2 || n > jobs || B->reads_singly) return false;
+    if (!B->read_jobs) {
+        B->read_slots += n;
+        if (B->read_slots < READ_AFTER) return false;
+        int64_t rows = 0;
+        for (const HostGroup &G : B->groups) rows += (int64_t)G.cap * G.N;
+        const int64_t stage = std::max(std::min(B->pool_cap, READ_STAGE), B->pmax_all);
+        const size_t at_w = (size_t)stage * sizeof(float4), at_jobs = at_w + (size_t)rows * sizeof(double);
+        const size_t bytes = at_jobs + (size_t)jobs * sizeof(psf::ReadJob);
+        unsigned char *p = nullptr;
+        double *host = nullptr;
+        if (cudaMalloc(&p, bytes) != cudaSuccess ||
+            cudaHostAlloc((void **)&host, (size_t)rows * 8, cudaHostAllocDefault) != cudaSuccess) {
             cudaGetLastError();
+            cudaFree(p);
+            B->reads_singly = true;
             return false;
         }
-        *cap = need;
-        B->bytes += need * (int64_t)unit;
-        return true;
-    };
-    if (n_w > B->read_host_cap) {
-        if (B->read_w_host) cudaFreeHost(B->read_w_host);
-        B->read_w_host = nullptr;
-        B->read_host_cap = 0;
-        if (cudaHostAlloc((void **)&B->read_w_host, (size_t)n_w * 8, cudaHostAllocDefault) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
-        B->read_host_cap = n_w;
+        B->read_stage = reinterpret_cast<float4 *>(p);
+        B->read_w = reinterpret_cast<double *>(p + at_w);
+        B->read_jobs = reinterpret_cast<psf::ReadJob *>(p + at_jobs);
+        B->read_w_host = host;
+        B->read_w_cap = rows;
+        B->read_stage_cap = stage;
+        B->bytes += (int64_t)bytes;
     }
-    const int64_t stage = std::min(n_parts, std::max(READ_STAGE, B->pmax_all));
-    return grow((void **)&B->read_w, &B->read_w_cap, n_w, sizeof(double)) &&
-           grow((void **)&B->read_jobs, &B->read_jobs_cap, jobs, sizeof(psf::ReadJob)) &&
-           grow((void **)&B->read_stage, &B->read_stage_cap, stage, sizeof(float4));
+    return n_w <= B->read_w_cap;
 }
 
 // Where the host memory that one copy may cover ends, starting from a host
@@ -1025,7 +1034,7 @@ int psf_batch_read_instances(psf_batch *B, int32_t n, const int32_t *basis, cons
     } catch (const std::bad_alloc &) {
         return fail(PSF_ERR_NOMEM, "host allocation failed");
     }
-    int64_t n_w = 0, n_parts = 0;
+    int64_t n_w = 0;
     for (int32_t i = 0; i < n; ++i) {
         int sg = 0;
         PSF_CHECK(slot_index(B, basis[i], slot[i], &sg));
@@ -1040,9 +1049,8 @@ int psf_batch_read_instances(psf_batch *B, int32_t n, const int32_t *basis, cons
         j.w_at = (int)n_w;
         j.n_parts = xyzw[i] ? (int)s.n_particles : 0;
         n_w += j.n_w;
-        n_parts += j.n_parts;
     }
-    if (n < 2 || n > 65535 || !prepare_read(B, n, n_w, n_parts)) return read_one_by_one(B, jobs, w, xyzw);
+    if (!group_read(B, n, n_w)) return read_one_by_one(B, jobs, w, xyzw);
     // Groups of slots that fill the staging buffer: [first, last).
     std::vector<std::pair<int32_t, int32_t>> groups;
     try {

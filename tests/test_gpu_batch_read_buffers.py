@@ -1,0 +1,50 @@
+"""Grouped read-back makes its buffers once, and not for a batch that is hardly read."""
+import numpy as np
+import pytest
+
+from parallelspectralfluids3d_b200 import _lib as L
+from parallelspectralfluids3d_b200.batch import Batch
+from parallelspectralfluids3d_b200.fixture import initial_coefficients, initial_particles
+from test_gpu_batch_read import read
+
+pytestmark = pytest.mark.gpu
+
+
+# Slots of two bases with counts below the staging, above it, and one slot that fills it.
+@pytest.mark.parametrize("counts", [(300, 0, 257, 1, 4096, 33, 512, 2), (1300000, 700, 1500000, 1400000), (40, 5000000)])
+def test_buffers_made_once(small_bases, counts):
+    bases = [small_bases["box576"], small_bases["sphere12x10x9"]]
+    params = L.make_params(dt=0.01, precision=L.PSF_PRECISION_BF16X2)
+    n = len(counts)
+    with Batch(bases, (n + 1) // 2, max(counts), autotune=False, particle_pool=sum(counts) + 256 * n) as bt:
+        where = [(k % 2, k // 2) for k in range(n)]
+        for k, (i, s) in enumerate(where):
+            b = bases[i]
+            bt.set_instance(i, s, initial_coefficients(b.n_modes, k), params,
+                            initial_particles(b, counts[k], k) if counts[k] else None)
+        bt.step(3)
+        want = [(bt.get_state(i, s), bt.get_particles(i, s)) for i, s in where]
+        flat = np.empty((sum(counts), 4), np.float32)
+        ends = np.cumsum(counts)
+        p = [flat[e - c:e] for c, e in zip(counts, ends)]
+        w = [np.empty(len(x[0])) for x in want]
+        sizes = [bt.info()["device_bytes"]]
+        asked = 0
+        while asked < 132:
+            m = 2 + asked % (n - 1)  # reads of every size
+            flat[:] = -7.0
+            for a in w:
+                a[:] = -7.0
+            L.check(read(bt, where[:m], w[:m], p[:m]))
+            asked += m
+            sizes.append(bt.info()["device_bytes"])
+            for k in range(n):
+                assert np.array_equal(w[k], want[k][0] if k < m else np.full(len(w[k]), -7.0))
+                assert np.array_equal(p[k], want[k][1]) if k < m else np.all(p[k] == -7.0)
+        assert sizes[1] == sizes[0]  # a first read of two slots makes none
+        assert len(set(sizes)) == 2 and sizes == sorted(sizes)
+        # The same slot more often than there are slots.
+        twice = [where[0]] * (2 * bt.slots[0] + 1)
+        q = [np.empty((counts[0], 4), np.float32) for _ in twice]
+        L.check(read(bt, twice, [None] * len(twice), q))
+        assert all(np.array_equal(a, want[0][1]) for a in q)
