@@ -167,8 +167,12 @@ constexpr int RUN_EXTRA = RUN_STEPS - 3;
 // A run's graph is captured once this many steps that could have gone into runs
 // were taken one by one.  Capturing and loading it takes 0.95 ms and a step in a
 // run is 2.2 to 6 us shorter, so about this many steps pay for it; a context
-// closed earlier pays nothing, and the latest to gain loses 1 ms once.
+// closed earlier pays nothing, and the latest to gain loses 1 ms once.  New
+// parameters or another number of particles drop the graphs: where their runs
+// had not paid for them by then, the next ones wait twice as long, so that a
+// program that changes its parameters every 320 steps does not lose 1 ms each time.
 constexpr int RUN_AFTER = 288;
+constexpr int RUN_AFTER_MOST = 1 << 24;
 
 struct psf_ctx {
     int device = 0;
@@ -182,6 +186,9 @@ struct psf_ctx {
     cudaGraph_t run_graphs[6] = {};             // RUN_STEPS steady steps, by the position they start from
     cudaGraphExec_t run_execs[6] = {};
     int singles = 0;                            // steps taken singly, since the last capture, that a run could have held
+    int run_after = RUN_AFTER;                  // ... at which the next run is captured
+    int runs_held = 0;                          // run graphs held
+    long long run_steps = 0;                    // steps taken in their runs
     double *wbuf[3 + RUN_EXTRA] = {};           // the ring, then the states between a run's first and last three
     unsigned long long *ctrbuf = nullptr;       // completed steps of each slot's state
     float *ubuf[2] = {nullptr, nullptr};
@@ -235,6 +242,11 @@ struct psf_ctx {
             run_execs[i] = nullptr;
             run_graphs[i] = nullptr;
         }
+        if (runs_held > 0)
+            run_after = run_steps >= (long long)runs_held * RUN_AFTER ? RUN_AFTER
+                                                                      : std::min(2 * run_after, RUN_AFTER_MOST);
+        runs_held = 0;
+        run_steps = 0;
         singles = 0;
     }
     int slot(int k) const { return (vis + k) % 3; }
@@ -452,11 +464,12 @@ static int capture_run(psf_ctx *c, int v, int q, cudaGraph_t *out)
 static int ready_run(psf_ctx *c, bool *ready)
 {
     const int idx = c->vis * 2 + c->tq;
-    if (!c->run_execs[idx] && c->singles >= RUN_AFTER) {
+    if (!c->run_execs[idx] && c->singles >= c->run_after) {
         cudaGraph_t g = nullptr;
         PSF_CHECK(capture_run(c, c->vis, c->tq, &g));
         c->run_graphs[idx] = g;
         PSF_CUDA(cudaGraphInstantiate(&c->run_execs[idx], g, 0));
+        ++c->runs_held;
         c->singles = 0;
     }
     *ready = c->run_execs[idx] != nullptr;
@@ -817,10 +830,12 @@ int psf_step(psf_ctx *c, int32_t nsteps)
             PSF_CHECK(ready_run(c, &run));
             if (!run) ++c->singles;
         }
-        if (run)
+        if (run) {
             PSF_CUDA(cudaGraphLaunch(c->run_execs[c->vis * 2 + c->tq], c->stream));
-        else
+            c->run_steps += RUN_STEPS;
+        } else {
             PSF_CHECK(launch_step(c));
+        }
         nsteps -= run ? RUN_STEPS : 1;
     }
     return PSF_OK;
