@@ -461,19 +461,25 @@ static int capture_run(psf_ctx *c, int v, int q, cudaGraph_t *out)
 // Whether RUN_STEPS steps of a primed pipeline can go in one launch from the
 // current ring position.  Where they cannot, single steps soon reach a position
 // that has its graph, as the six positions follow one another.
-static int ready_run(psf_ctx *c, bool *ready)
+static bool ready_run(psf_ctx *c)
 {
     const int idx = c->vis * 2 + c->tq;
     if (!c->run_execs[idx] && c->singles >= c->run_after) {
         cudaGraph_t g = nullptr;
-        PSF_CHECK(capture_run(c, c->vis, c->tq, &g));
-        c->run_graphs[idx] = g;
-        PSF_CUDA(cudaGraphInstantiate(&c->run_execs[idx], g, 0));
-        ++c->runs_held;
         c->singles = 0;
+        if (capture_run(c, c->vis, c->tq, &g) == PSF_OK &&
+            cudaGraphInstantiate(&c->run_execs[idx], g, 0) == cudaSuccess) {
+            c->run_graphs[idx] = g;
+            ++c->runs_held;
+        } else {
+            // No memory for a run: the steps go on one by one.
+            cudaGetLastError();
+            if (g) cudaGraphDestroy(g);
+            c->run_execs[idx] = nullptr;
+            c->run_after = RUN_AFTER_MOST;
+        }
     }
-    *ready = c->run_execs[idx] != nullptr;
-    return PSF_OK;
+    return c->run_execs[idx] != nullptr;
 }
 
 // Launch one step and rotate the ring.  A kind's six ring positions are captured
@@ -827,7 +833,7 @@ int psf_step(psf_ctx *c, int32_t nsteps)
     while (nsteps > 0) {
         bool run = false;
         if (c->primed && nsteps >= RUN_STEPS) {
-            PSF_CHECK(ready_run(c, &run));
+            run = ready_run(c);
             if (!run) ++c->singles;
         }
         if (run) {

@@ -129,6 +129,8 @@ struct psf_batch {
     cudaStream_t stream = nullptr;
     cudaGraph_t graphs[2] = {nullptr, nullptr};      // one step, RUN_STEPS steps
     cudaGraphExec_t execs[2] = {nullptr, nullptr};
+    int64_t singles = 0;                             // steps taken singly
+    bool no_run = false;                             // no memory for the longer graph
     std::vector<HostGroup> groups;
     std::vector<psf::SlotDev> slots;  // host mirror of the slot table
     std::vector<long long> prefix;  // host copy of the tracer's slot prefix sums
@@ -652,8 +654,11 @@ int launch_step(psf_batch *B, cudaStream_t st, bool after_kernel)
 // 384 158.7 -> 156.  The tracer does not start this way: its blocks would come
 // up beside the reconstruction's, on SMs set to a small L1 (64 of N = 384:
 // 184 us).  Nor the state update, whose blocks hold up the contraction's end
-// (67.5 us for 40 of N = 200).
+// (67.5 us for 40 of N = 200).  Capturing it costs 30 us more than the graph of
+// one step, so a batch that has taken and is asked for fewer than RUN_PAYS steps
+// does without (a new batch's first 8 steps: 329 us, with it 360).
 constexpr int RUN_STEPS = 8;
+constexpr int RUN_PAYS = 2 * RUN_STEPS;
 
 // Steps between two looks at the particles' order (psf_batch_reorder).
 constexpr int ORDER_EVERY = 64;
@@ -671,8 +676,13 @@ int build_graph(psf_batch *B, int which)
         return rc;
     }
     if (e != cudaSuccess) return psf::cuda_fail(e, "cudaStreamEndCapture");
+    e = cudaGraphInstantiate(&B->execs[which], g, 0);
+    if (e != cudaSuccess) {
+        cudaGraphDestroy(g);
+        B->execs[which] = nullptr;
+        return psf::cuda_fail(e, "cudaGraphInstantiate");
+    }
     B->graphs[which] = g;
-    PSF_CUDA(cudaGraphInstantiate(&B->execs[which], g, 0));
     return PSF_OK;
 }
 
@@ -1119,8 +1129,19 @@ int psf_batch_step(psf_batch *B, int32_t nsteps)
     if (nsteps < 0) return fail(PSF_ERR_INVALID, "nsteps must be >= 0");
     PSF_CUDA(cudaSetDevice(B->device));
     while (nsteps > 0) {
-        const int which = nsteps >= RUN_STEPS ? 1 : 0;
-        PSF_CHECK(build_graph(B, which));
+        int which = 0;
+        if (nsteps >= RUN_STEPS && !B->no_run && (B->execs[1] || B->singles + (int64_t)nsteps >= RUN_PAYS)) {
+            if (build_graph(B, 1) == PSF_OK) {
+                which = 1;
+            } else {  // no memory for it: the steps go on one by one
+                cudaGetLastError();
+                B->no_run = true;
+            }
+        }
+        if (which == 0) {
+            PSF_CHECK(build_graph(B, 0));
+            ++B->singles;
+        }
         PSF_CUDA(cudaGraphLaunch(B->execs[which], B->stream));
         const int taken = which ? RUN_STEPS : 1;
         nsteps -= taken;
