@@ -374,8 +374,26 @@ struct WedgePlan {
     size_t w_bytes, partial_bytes;
 };
 
-WedgePlan plan_of(const psf_wedge_desc *d, int k0, int kb)
+// What the workspace of batches of k_batch modes may take: W with all ldn columns
+// of a mode and its partial sums over so many splits that 128 x 128 tiles of them
+// come to about two per SM, which is what it took before half of the columns were
+// left out: N = 512 in batches of 8 modes (5,000 edges) would take 258 MB instead
+// of 214 otherwise.  Fewer splits cost up to 13 % there (16^3, N = 512: 60.5 against
+// 53.6 ms, with all columns 149 ms); up to N = 256 in batches of 64 modes the bound
+// changes nothing.
+size_t workspace_bound(const psf_wedge_desc *d, int k_batch)
 {
+    const long long chunks = (d->n_edges + GB_K - 1) / GB_K, ldc = (long long)k_batch * d->ldn;
+    const long long tiles = (long long)(d->ldn / 128) * (ldc / 128);
+    long long splits = std::max(1ll, std::min({(2ll * 148 + tiles - 1) / tiles, 64ll, std::max(1ll, chunks)}));
+    const long long per = std::max(1ll, (chunks + splits - 1) / splits);
+    splits = std::max(1ll, (chunks + per - 1) / per);
+    return (size_t)(chunks * GB_K + splits * d->ldn) * ldc * sizeof(double);
+}
+
+WedgePlan plan_of(const psf_wedge_desc *d, int k_batch, int k0)
+{
+    const int kb = std::min(k_batch, d->n_modes - k0);
     WedgePlan p{};
     p.n_chunks = (d->n_edges + GB_K - 1) / GB_K;
     p.rows = p.n_chunks * GB_K;
@@ -383,6 +401,11 @@ WedgePlan plan_of(const psf_wedge_desc *d, int k0, int kb)
     p.ldc = p.col_tiles * GB_N;
     p.row_tiles = (d->n_modes + GB_M - 1) / GB_M;
     const long long tiles = p.row_tiles * p.col_tiles, slots = 148ll * GB_PER_SM;
+    p.w_bytes = (size_t)p.rows * p.ldc * sizeof(double);
+    // The partial sums follow the W of the first batch, the largest.
+    const long long ldc0 = (columns_before(d->n_modes, 0, k_batch) + GB_N - 1) / GB_N * GB_N;
+    const size_t split_bytes = (size_t)p.row_tiles * GB_M * p.ldc * sizeof(double);
+    const long long most = (long long)((workspace_bound(d, k_batch) - (size_t)p.rows * ldc0 * sizeof(double)) / split_bytes);
     double best = 1e300;
     p.splits = p.chunks_per_split = 1;
     for (long long s = 1; s <= std::min(64ll, std::max(1ll, p.n_chunks)); ++s) {
@@ -390,14 +413,13 @@ WedgePlan plan_of(const psf_wedge_desc *d, int k0, int kb)
         const long long used = std::max(1ll, (p.n_chunks + per - 1) / per);
         const double cost = (double)((tiles * used + slots - 1) / slots) * (double)(per + 8) * 2.4 +
                             (double)used * (double)(tiles * GB_M * GB_N * 16) / 5e6;
-        if (cost < best) {
+        if (cost < best && used <= std::max(1ll, most)) {
             best = cost;
             p.splits = used;
             p.chunks_per_split = per;
         }
     }
-    p.w_bytes = (size_t)p.rows * p.ldc * sizeof(double);
-    p.partial_bytes = (size_t)p.splits * p.row_tiles * GB_M * p.ldc * sizeof(double);
+    p.partial_bytes = (size_t)p.splits * split_bytes;
     return p;
 }
 
@@ -411,7 +433,7 @@ Workspace workspace_of(const psf_wedge_desc *d, int kb)
 {
     Workspace ws{0, 0};
     for (int k0 = 0; k0 < d->n_modes; k0 += kb) {
-        const WedgePlan q = plan_of(d, k0, std::min(kb, d->n_modes - k0));
+        const WedgePlan q = plan_of(d, kb, k0);
         ws.w_bytes = std::max(ws.w_bytes, q.w_bytes);
         ws.partial_bytes = std::max(ws.partial_bytes, q.partial_bytes);
     }
@@ -495,7 +517,7 @@ extern "C" int psf_pre_advection_tensor(const psf_wedge_desc *d, int32_t k_batch
     const int N = d->n_modes;
     for (int k0 = 0; k0 < N; k0 += k_batch) {
         const int kb = std::min(k_batch, N - k0);
-        const WedgePlan q = plan_of(d, k0, kb);
+        const WedgePlan q = plan_of(d, k_batch, k0);
         const long long wblocks = std::max(1ll, std::min<long long>((q.rows + 7) / 8, 148ll * 16));
         psf_wedge_w<<<(unsigned)wblocks, 256, 0, st>>>(d->n_edges, q.rows, N, d->ldn, q.ldc, k0, kb, d->edge_faces,
                                                        d->edge_S, d->phi, d->phi_zero_row, W);
