@@ -2,19 +2,28 @@
 // reference's PSFSolverGPU::drawParticles (Solver/SolverImpl/psfsolvergpu.cpp:876-1022)
 // as CUDA kernels writing device buffers, with no graphics API.
 //
+//   psf_vol_clear      zeroes what the last frame left (Texture3D::clearImage)
 //   psf_vol_histogram  particle -> cell counts; a warp merges equal cells
 //                      (__match_any_sync) before one atomic per distinct cell
-//   psf_vol_density    counts / 1e6 -> FP16 density, clears the counts for the
-//                      next frame (volume.comp, Texture3D::clearImage) and
-//                      notes which texels are not zero, one bit each
+//   psf_vol_density    counts / 1e6 -> FP16 density (volume.comp) in the counts'
+//                      place, and one bit for every texel that is not zero
 //   psf_vol_occupancy  one bit per trilinear cell: any of its 8 texels not zero
+//   psf_vol_unpack     the density as res^3 FP16 values, for reading back
 //   psf_vol_render     a lane carries one ray at a time: ray/AABB slab test,
 //                      march with trilinear clamp-to-border samples, shadow ray
 //                      toward the light, front-to-back emission/absorption
 //                      (volume.frag); cells without density are stepped over
 //
-// The density (R^3 FP16, 32 MB at R = 256) stays L2-resident while a frame is
-// rendered.  Arithmetic is round-to-nearest FP32 through explicit intrinsics
+// A volume is one array of 4-byte words, R + 2 slices of R + 2 rows of R + 1
+// words, and the bits.  Word c of the row of texels (y, z), row y + 1 of slice
+// z + 1, holds the texels (c - 1, c) as two FP16 values; the outer rows and
+// slices are the zero border.  While particles are counted, word c of that row
+// holds the count of texel c.  So a sample of the march is four loads with no
+// border tests, and a volume takes 4.3 bytes per texel (571 MB at R = 512; the
+// counts and an FP16 array beside them would be 805 MB).
+//
+// The density (68 MB at R = 256) stays L2-resident while a frame is rendered.
+// Arithmetic is round-to-nearest FP32 through explicit intrinsics
 // in a fixed order (no contraction), so results equal a plain C restatement
 // bit for bit.
 #include <cuda_fp16.h>
@@ -27,6 +36,7 @@
 #include <new>
 #include <string>
 
+#include "psf_device.cuh"
 #include "psf_internal.h"
 #include "psf_volume.h"
 
@@ -47,77 +57,108 @@ struct View {
     int W, H, R;
 };
 
-// Grid-stride over groups of 32 particles so every lane takes part in the match.
-__global__ void psf_vol_histogram(const float4 *__restrict__ p, long long n, Box b, int *__restrict__ hist)
+// Words from a row to the next and from a slice to the next.
+__host__ __device__ __forceinline__ uint32_t row_pitch(int R) { return (uint32_t)R + 1u; }
+__host__ __device__ __forceinline__ uint32_t slice_pitch(int R) { return ((uint32_t)R + 1u) * ((uint32_t)R + 2u); }
+// First word of the row of texels (y, z).
+__host__ __device__ __forceinline__ uint32_t row_at(int R, uint32_t y, uint32_t z)
 {
+    return (z + 1u) * slice_pitch(R) + (y + 1u) * row_pitch(R);
+}
+uint32_t row_words_of(int R) { return (uint32_t)(R + 31) / 32; }       // bit words of a row of texels
+uint32_t cell_words_of(int R) { return (uint32_t)(R + 1 + 31) / 32; }  // ... and of cells
+
+// The kernels of a splat start during the tail of the one before (programmatic
+// dependent launch): 10.6 us for all four at R = 64 with 1,000 particles.
+
+// Zeroes the words that hold density: those of a texel with its bit set and of the
+// texel after it.  A warp takes a row.
+__global__ void __launch_bounds__(256) psf_vol_clear(uint32_t *__restrict__ words,
+                                                     const uint32_t *__restrict__ texel_bits, int R, int row_words)
+{
+    const int lane = threadIdx.x & 31;
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+    psf::launch_dependents();
+    for (uint32_t row = warp; row < (uint32_t)R * (uint32_t)R; row += nwarps) {
+        const uint32_t mine = lane < row_words ? texel_bits[(size_t)row * row_words + lane] : 0u;
+        if (!__any_sync(0xffffffffu, mine != 0u)) continue;
+        uint32_t *w = words + row_at(R, row % (uint32_t)R, row / (uint32_t)R);
+        uint32_t carry = 0;
+        for (int k = 0; k * 32 <= R; ++k) {
+            const uint32_t m = k < row_words ? __shfl_sync(0xffffffffu, mine, k) : 0u;
+            const uint32_t held = m | (m << 1) | carry;
+            carry = m >> 31;
+            const int c = k * 32 + lane;
+            if (c <= R && ((held >> lane) & 1u)) w[c] = 0u;
+        }
+    }
+}
+
+// Grid-stride over groups of 32 particles so every lane takes part in the match.
+__global__ void psf_vol_histogram(const float4 *__restrict__ p, long long n, Box b, int *__restrict__ words)
+{
+    psf::grid_dependency_wait();
+    psf::launch_dependents();
     const int lane = threadIdx.x & 31;
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
     for (long long base = warp * 32; base < n; base += nwarps * 32) {
         const long long i = base + lane;
-        long long key = -1;
+        int key = -1;
         if (i < n) {
             const float4 q = p[i];
             const float c[3] = {q.x, q.y, q.z};
-            long long idx = 0;
+            uint32_t at[3];
             bool ok = true;
-            for (int a = 2; a >= 0; --a) {
+            for (int a = 0; a < 3; ++a) {
                 const float t = __fdiv_rn(__fsub_rn(c[a], b.mn[a]), b.ext[a]);
                 const float f = floorf(__fmul_rn(t, (float)b.R));
                 if (!(f >= 0.0f) || f >= (float)b.R) ok = false;
-                else idx = idx * b.R + (long long)f;
+                at[a] = ok ? (uint32_t)f : 0u;
             }
-            if (ok) key = idx;
+            if (ok) key = (int)(row_at(b.R, at[1], at[2]) + at[0]);
         }
         const unsigned same = __match_any_sync(0xffffffffu, key);
-        if (key >= 0 && lane == __ffs(same) - 1) atomicAdd(hist + key, __popc(same));
+        if (key >= 0 && lane == __ffs(same) - 1) atomicAdd(words + key, __popc(same));
     }
 }
 
-// A warp takes a row of texels, four words of 32 with their loads in flight.
-// It writes the density twice: as the texels and as the pairs the ray march
-// reads, pairs[z + 1][y + 1][c] = (texel c - 1, texel c) with c in [0, R]
-// (the rows y or z = -1 and R stay zero from the allocation).  Traffic bounds
-// it: 4 B read and 6 B written per texel; a count is cleared only where there
-// is one.
-__global__ void __launch_bounds__(256) psf_vol_density(int *__restrict__ hist, __half *__restrict__ vol,
-                                                       __half2 *__restrict__ pairs,
-                                                       uint32_t *__restrict__ texel_bits, int R, int row_words)
+// A warp takes a row of texels, four runs of 32 with their loads in flight.  A
+// word is read and written by the same lane, so the density takes the place of
+// the counts; words of empty cells are zero already and are not written.  Traffic
+// bounds it: 4 B read per texel, and 4 B written here and in psf_vol_clear where
+// there is density.  Splat of 2 M particles over 256^3 82 us, of 100,000 56 (with
+// counts, FP16 array and pairs apart 103 and 62; counts and FP16 array 84 and 56).
+__global__ void __launch_bounds__(256) psf_vol_density(uint32_t *__restrict__ words, uint32_t *__restrict__ texel_bits,
+                                                       int R, int row_words)
 {
+    psf::grid_dependency_wait();
+    psf::launch_dependents();
     const int lane = threadIdx.x & 31;
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-    const __half zero = __ushort_as_half((unsigned short)0);
     for (uint32_t row = warp; row < (uint32_t)R * (uint32_t)R; row += nwarps) {
-        int *hr = hist + (size_t)row * R;
-        __half *vr = vol + (size_t)row * R;
-        const uint32_t y = row % (uint32_t)R, z = row / (uint32_t)R;
-        __half2 *pr = pairs + ((size_t)(z + 1) * (R + 2) + (y + 1)) * (R + 1);
-        __half before = zero;
+        uint32_t *w = words + row_at(R, row % (uint32_t)R, row / (uint32_t)R);
+        uint32_t before = 0;
         for (int w0 = 0; w0 < row_words; w0 += 4) {
-            int h[4];
+            uint32_t h[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const int x = (w0 + k) * 32 + lane;
-                h[k] = x < R ? hr[x] : 0;
+                h[k] = x < R ? w[x] : 0u;
             }
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const int x = (w0 + k) * 32 + lane;
-                __half d = zero;
-                if (h[k]) {
-                    d = __float2half_rn(__fdiv_rn((float)h[k], 1000000.0f));
-                    hr[x] = 0;
-                }
-                const __half up = __shfl_up_sync(0xffffffffu, d, 1);
-                const __half prev = lane == 0 ? before : up;
+                const uint32_t d =
+                    h[k] ? (uint32_t)__half_as_ushort(__float2half_rn(__fdiv_rn((float)(int)h[k], 1000000.0f))) : 0u;
+                const uint32_t up = __shfl_up_sync(0xffffffffu, d, 1);
+                const uint32_t pair = (lane == 0 ? before : up) | (d << 16);
                 before = __shfl_sync(0xffffffffu, d, 31);
-                if (x < R) {
-                    vr[x] = d;
-                    pr[x] = __halves2half2(prev, d);
-                    if (x == R - 1) pr[R] = __halves2half2(d, zero);
-                }
-                const uint32_t bits = __ballot_sync(0xffffffffu, __half_as_ushort(d) != 0);
+                if (x < R && pair) w[x] = pair;
+                if (x == R - 1 && d) w[R] = d;
+                const uint32_t bits = __ballot_sync(0xffffffffu, d != 0u);
                 if (lane == 0 && w0 + k < row_words) texel_bits[(size_t)row * row_words + w0 + k] = bits;
             }
         }
@@ -130,6 +171,7 @@ __global__ void __launch_bounds__(256) psf_vol_occupancy(const uint32_t *__restr
                                                          uint32_t row_words, uint32_t cell_words, uint32_t words,
                                                          uint32_t *__restrict__ cell_bits)
 {
+    psf::grid_dependency_wait();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= words) return;
     const uint32_t w = t % cell_words, row = t / cell_words;
@@ -142,6 +184,16 @@ __global__ void __launch_bounds__(256) psf_vol_occupancy(const uint32_t *__restr
             if (w > 0) before |= b[w - 1];
         }
     cell_bits[t] = here | (here << 1) | (before >> 31);
+}
+
+// Texels of the slices from z0 on.
+__global__ void __launch_bounds__(256) psf_vol_unpack(const uint32_t *__restrict__ words, int R, uint32_t z0,
+                                                      uint32_t texels, uint16_t *__restrict__ out)
+{
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= texels) return;
+    const uint32_t row = t / (uint32_t)R, x = t % (uint32_t)R;
+    out[t] = (uint16_t)(words[row_at(R, row % (uint32_t)R, z0 + row / (uint32_t)R) + x] >> 16);
 }
 
 __device__ __forceinline__ float lerp1(float a, float b, float t)
@@ -166,9 +218,7 @@ __device__ __forceinline__ bool in_border(float u, float v, float w, float Rf)
     return u >= -1.0f && u < Rf && v >= -1.0f && v < Rf && w >= -1.0f && w < Rf;
 }
 
-// Trilinear clamp-to-border sample.  `pairs` holds, for every cell c along x
-// and every texel row with one border row around them, the texels (c - 1, c):
-// a sample is four 4-byte loads with no border tests.
+// Trilinear clamp-to-border sample: four 4-byte loads with no border tests.
 __device__ __forceinline__ float sample(const __half2 *__restrict__ pairs, int R, float px, float py, float pz)
 {
     const float Rf = (float)R;
@@ -177,7 +227,7 @@ __device__ __forceinline__ float sample(const __half2 *__restrict__ pairs, int R
     float fu, fv, fw;
     const uint32_t ux = floor_cell(u, fu), uy = floor_cell(v, fv), uz = floor_cell(w, fw);
     const float a = __fsub_rn(u, fu), b = __fsub_rn(v, fv), c = __fsub_rn(w, fw);
-    const uint32_t row = (uint32_t)(R + 1), slice = row * (uint32_t)(R + 2);
+    const uint32_t row = row_pitch(R), slice = slice_pitch(R);
     const __half2 *at = pairs + (uz * slice + uy * row + ux);
     const float2 t00 = __half22float2(__ldg(at)), t10 = __half22float2(__ldg(at + row));
     const float2 t01 = __half22float2(__ldg(at + slice)), t11 = __half22float2(__ldg(at + slice + row));
@@ -534,11 +584,11 @@ struct psf_volume {
     int sms = 148;
     int R = 256;
     cudaStream_t stream = nullptr;  // own stream (host splats and renders)
-    int *hist = nullptr;
-    __half *vol = nullptr;
-    __half2 *pairs = nullptr;       // x-neighbour pairs with zero border rows, read by the ray march
+    uint32_t *words = nullptr;      // counts, then pairs of texels; the rest follows in the same allocation
     uint32_t *texel_bits = nullptr, *cell_bits = nullptr;  // occupancy of texels and of trilinear cells
     uint32_t *next = nullptr;       // the ray march's pixel counter
+    uint16_t *texels = nullptr;     // slices of the density on their way to the host
+    int texel_slices = 1;
     int render_blocks = 148 * 4;
     float4 *parts = nullptr;        // host-splat staging
     long long parts_cap = 0;
@@ -576,24 +626,29 @@ int make_box(const float *mn, const float *mx, int R, Box *b)
     return PSF_OK;
 }
 
-uint32_t row_words_of(int R) { return (uint32_t)(R + 31) / 32; }       // texels of a row
-uint32_t cell_words_of(int R) { return (uint32_t)(R + 1 + 31) / 32; }  // cells of a row
-
 int launch_splat(psf_volume *v, const float4 *parts, long long n, const Box &b, cudaStream_t st)
 {
-    if (n > 0) {
-        const long long need = (n + 255) / 256;
-        const int grid = (int)std::max<long long>(1, std::min<long long>(need, (long long)v->sms * 8));
-        psf_vol_histogram<<<grid, 256, 0, st>>>(parts, n, b, v->hist);
-    }
     const uint32_t row_words = row_words_of(v->R), cell_words = cell_words_of(v->R);
     const uint32_t rows = (uint32_t)v->R * (uint32_t)v->R;
-    const int grid = (int)std::min<long long>((rows + 7) / 8, (long long)v->sms * 8);
-    psf_vol_density<<<grid, 256, 0, st>>>(v->hist, v->vol, v->pairs, v->texel_bits, v->R, (int)row_words);
-    const uint32_t owords = (uint32_t)(v->R + 1) * (uint32_t)(v->R + 1) * cell_words;
-    psf_vol_occupancy<<<(owords + 255) / 256, 256, 0, st>>>(v->texel_bits, v->R, row_words, cell_words, owords,
-                                                           v->cell_bits);
-    return cuda_status(cudaGetLastError(), "volume splat launch");
+    const unsigned grid = (unsigned)std::min<long long>((rows + 7) / 8, (long long)v->sms * 8);
+    psf_vol_clear<<<grid, 256, 0, st>>>(v->words, v->texel_bits, v->R, (int)row_words);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess && n > 0) {
+        const unsigned blocks = (unsigned)std::min<long long>((n + 255) / 256, (long long)v->sms * 8);
+        psf::PdlLaunch L(blocks, 256, st, /*after_kernel=*/true);
+        e = cudaLaunchKernelEx(&L.cfg, psf_vol_histogram, parts, n, b, reinterpret_cast<int *>(v->words));
+    }
+    if (e == cudaSuccess) {
+        psf::PdlLaunch L(grid, 256, st, /*after_kernel=*/true);
+        e = cudaLaunchKernelEx(&L.cfg, psf_vol_density, v->words, v->texel_bits, (int)v->R, (int)row_words);
+    }
+    if (e == cudaSuccess) {
+        const uint32_t owords = (uint32_t)(v->R + 1) * (uint32_t)(v->R + 1) * cell_words;
+        psf::PdlLaunch L((owords + 255) / 256, 256, st, /*after_kernel=*/true);
+        e = cudaLaunchKernelEx(&L.cfg, psf_vol_occupancy, (const uint32_t *)v->texel_bits, (int)v->R, row_words,
+                               cell_words, owords, v->cell_bits);
+    }
+    return cuda_status(e, "volume splat launch");
 }
 
 int check_view(const psf_volume_view *view)
@@ -630,7 +685,7 @@ int launch_render(psf_volume *v, const psf_volume_view *view, cudaStream_t st)
     const long long warps = (long long)v->render_blocks * (RENDER_THREADS / 32);
     const int hold = (int)std::max<long long>(4, std::min<long long>(32, items / (warps * HANDS)));
     psf_vol_render<<<(unsigned)std::min<long long>(need, v->render_blocks), RENDER_THREADS, 0, st>>>(
-        v->pairs, v->cell_bits, cell_words_of(v->R), V, tiles_x, (uint32_t)items, hold, v->next, v->img);
+        reinterpret_cast<const __half2 *>(v->words), v->cell_bits, cell_words_of(v->R), V, tiles_x, (uint32_t)items, hold, v->next, v->img);
     return cuda_status(cudaGetLastError(), "volume render launch");
 }
 
@@ -663,23 +718,24 @@ int psf_volume_create(int device, int32_t res, psf_volume **out)
     v->device = device;
     v->R = res;
     cudaDeviceGetAttribute(&v->sms, cudaDevAttrMultiProcessorCount, device);
-    const size_t cells = (size_t)res * res * res;
     cudaError_t e = cudaStreamCreateWithFlags(&v->stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMalloc(&v->hist, cells * sizeof(int));
-    if (e == cudaSuccess) e = cudaMalloc(&v->vol, cells * sizeof(__half));
+    const size_t words = (size_t)(res + 2) * slice_pitch(res);
     const size_t tw = (size_t)res * res * row_words_of(res), cw = (size_t)(res + 1) * (res + 1) * cell_words_of(res);
-    if (e == cudaSuccess) e = cudaMalloc(&v->texel_bits, tw * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&v->cell_bits, cw * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&v->next, sizeof(uint32_t));
-    const size_t np = (size_t)(res + 2) * (res + 2) * (res + 1);
-    if (e == cudaSuccess) e = cudaMalloc(&v->pairs, np * sizeof(__half2));
-    if (e == cudaSuccess) e = cudaMemsetAsync(v->pairs, 0, np * sizeof(__half2), v->stream);
+    // Half of the density at a time crosses to the host, or 16 MB.
+    v->texel_slices = (int)std::max<size_t>(1, std::min<size_t>((res + 1) / 2, (8u << 20) / ((size_t)res * res)));
+    const size_t staging = (size_t)v->texel_slices * res * res;
+    if (e == cudaSuccess) e = cudaMalloc(&v->words, (words + tw + cw + 1) * sizeof(uint32_t) + staging * sizeof(uint16_t));
+    if (e == cudaSuccess) {
+        v->texel_bits = v->words + words;
+        v->cell_bits = v->texel_bits + tw;
+        v->next = v->cell_bits + cw;
+        v->texels = reinterpret_cast<uint16_t *>(v->next + 1);
+        e = cudaMemsetAsync(v->words, 0, (words + tw + cw) * sizeof(uint32_t), v->stream);
+    }
     int per_sm = 0;
     if (e == cudaSuccess)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, psf_vol_render, RENDER_THREADS, 0);
     if (e == cudaSuccess) v->render_blocks = v->sms * std::max(1, per_sm);
-    if (e == cudaSuccess) e = cudaMemsetAsync(v->hist, 0, cells * sizeof(int), v->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(v->vol, 0, cells * sizeof(__half), v->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(v->stream);
     if (e != cudaSuccess) {
         psf_volume_destroy(v);
@@ -694,12 +750,7 @@ int psf_volume_destroy(psf_volume *v)
     if (!v) return psf::fail(PSF_ERR_INVALID, "null volume");
     cudaSetDevice(v->device);
     if (v->stream) cudaStreamSynchronize(v->stream);
-    cudaFree(v->hist);
-    cudaFree(v->vol);
-    cudaFree(v->pairs);
-    cudaFree(v->texel_bits);
-    cudaFree(v->cell_bits);
-    cudaFree(v->next);
+    cudaFree(v->words);
     cudaFree(v->parts);
     cudaFree(v->img);
     if (v->stream) cudaStreamDestroy(v->stream);
@@ -775,7 +826,15 @@ int psf_volume_get_density(psf_volume *v, uint16_t *density, int64_t count)
     if (count < cells) return psf::fail(PSF_ERR_INVALID, "output smaller than res^3");
     const cudaError_t es = cudaSetDevice(v->device);
     if (es != cudaSuccess) return psf::cuda_fail(es, "cudaSetDevice");
-    cudaError_t e = cudaMemcpyAsync(density, v->vol, (size_t)cells * sizeof(__half), cudaMemcpyDeviceToHost, v->stream);
+    const size_t slice = (size_t)v->R * v->R;
+    cudaError_t e = cudaSuccess;
+    for (int z = 0; z < v->R && e == cudaSuccess; z += v->texel_slices) {
+        const uint32_t texels = (uint32_t)(slice * std::min(v->texel_slices, v->R - z));
+        psf_vol_unpack<<<(texels + 255) / 256, 256, 0, v->stream>>>(v->words, v->R, (uint32_t)z, texels, v->texels);
+        e = cudaGetLastError();
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(density + slice * z, v->texels, texels * sizeof(uint16_t), cudaMemcpyDeviceToHost, v->stream);
+    }
     if (e == cudaSuccess) e = cudaStreamSynchronize(v->stream);
     return cuda_status(e, "density read-back");
 }
