@@ -116,6 +116,10 @@ int psf_batch_get_particles(psf_batch *b, int32_t basis, int32_t slot, float *xy
  * particles were last traced with; none before a slot's first step). */
 int psf_batch_get_velocity(psf_batch *b, int32_t basis, int32_t slot, float *u, int64_t n_faces);
 int psf_batch_get_steps(psf_batch *b, int32_t basis, int32_t slot, int64_t *steps);
+/* Slots whose particles the last look at the particles' storage order found
+ * mixed by the flow and put back (psf_batch_step looks every 64 steps; nothing
+ * else shows the order).  0 before the first look. */
+int psf_batch_get_reordered(psf_batch *b, int32_t *slots);
 
 /* One step, run as psf_batch_step runs it, with each launch timed between
  * CUDA events (milliseconds): [tensor-core step, tracer] for a fused batch,

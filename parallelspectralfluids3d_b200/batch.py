@@ -209,3 +209,9 @@ class Batch:
         s = ct.c_int64()
         L.check(self.lib.psf_batch_get_steps(self.handle, int(basis), int(slot), ct.byref(s)))
         return int(s.value)
+
+    def get_reordered(self) -> int:
+        """Slots whose particles the last look (every 64 steps) found mixed and put back in order."""
+        n = ct.c_int32()
+        L.check(self.lib.psf_batch_get_reordered(self.handle, ct.byref(n)))
+        return int(n.value)

@@ -1229,6 +1229,24 @@ int psf_batch_get_velocity(psf_batch *B, int32_t basis, int32_t slot, float *u, 
     return check_device_error(B);
 }
 
+int psf_batch_get_reordered(psf_batch *B, int32_t *slots)
+{
+    if (!B || !slots) return fail(PSF_ERR_INVALID, "null argument");
+    PSF_CUDA(cudaSetDevice(B->device));
+    std::vector<psf::SlotDev> now;
+    try {
+        now.resize(B->slots.size());
+    } catch (const std::bad_alloc &) {
+        return fail(PSF_ERR_NOMEM, "host allocation failed");
+    }
+    PSF_CUDA(cudaMemcpyAsync(now.data(), B->d_slots, now.size() * sizeof(psf::SlotDev), cudaMemcpyDeviceToHost,
+                             B->stream));
+    PSF_CUDA(cudaStreamSynchronize(B->stream));
+    *slots = 0;
+    for (const psf::SlotDev &s : now) *slots += B->order_round > 0 && s.mixed == B->order_round;
+    return PSF_OK;
+}
+
 int psf_batch_get_steps(psf_batch *B, int32_t basis, int32_t slot, int64_t *steps)
 {
     int sg = 0;
