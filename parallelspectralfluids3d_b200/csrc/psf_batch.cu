@@ -512,8 +512,7 @@ __global__ void __launch_bounds__(256) psf_batch_state(const GroupDev *__restric
 {
     __shared__ double red[8];
     __shared__ double wnew[PSF_MAX_MODES];
-    grid_dependency_wait();
-    launch_dependents();
+    launch_dependents();  // the reconstruction, which waits for this grid's end before it reads
     SlotDev &s = slots[blockIdx.x];
     if (!s.active) return;
     if (s.target != 0ull && s.step >= s.target) {
@@ -651,8 +650,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK, 5) psf_batch_trace(const GroupDev
     __shared__ uint32_t aside_at[ASIDE ? TRACE_BLOCK / 32 : 1][64];
     for (int i = threadIdx.x; i <= n_slots; i += blockDim.x) pre[i] = prefix[i];
     __syncthreads();
-    grid_dependency_wait();
-    launch_dependents();
+    launch_dependents();  // the next step's contraction, which waits for this grid's end
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int32_t *as = aside_slot[ASIDE ? warp : 0];
     uint32_t *aa = aside_at[ASIDE ? warp : 0];
@@ -985,11 +983,11 @@ int max_fused_grid(int bn_max, int num_sms)
     return per_sm * num_sms;
 }
 
-int launch_batch_state(const GroupDev *groups, SlotDev *slots, int n_slots, cudaStream_t st, bool after_kernel)
+int launch_batch_state(const GroupDev *groups, SlotDev *slots, int n_slots, cudaStream_t st)
 {
     if (n_slots <= 0) return PSF_OK;
-    PdlLaunch L((unsigned)n_slots, 256, st, after_kernel);
-    cudaError_t e = cudaLaunchKernelEx(&L.cfg, psf_batch_state, groups, slots);
+    psf_batch_state<<<n_slots, 256, 0, st>>>(groups, slots);
+    cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? PSF_OK : cuda_fail(e, "psf_batch_state launch");
 }
 
@@ -1029,15 +1027,14 @@ int batch_trace_grid(int num_sms, bool faces)
 }
 
 int launch_batch_trace(const GroupDev *groups, const SlotDev *slots, const long long *prefix, int n_slots, int grid,
-                       bool all_centred, bool faces, cudaStream_t st, bool after_kernel)
+                       bool all_centred, bool faces, cudaStream_t st)
 {
     if (n_slots < 1 || n_slots > BATCH_MAX_ALL_SLOTS) return fail(PSF_ERR_INVALID, "slot count out of range");
-    PdlLaunch L((unsigned)grid, TRACE_BLOCK, st, after_kernel);
-    cudaError_t e = cudaLaunchKernelEx(&L.cfg,
-                                       faces         ? psf_batch_trace<true, true>
-                                       : all_centred ? psf_batch_trace<true, false>
-                                                     : psf_batch_trace<false, false>,
-                                       groups, slots, prefix, n_slots);
+    auto kernel = faces         ? psf_batch_trace<true, true>
+                  : all_centred ? psf_batch_trace<true, false>
+                                : psf_batch_trace<false, false>;
+    kernel<<<grid, TRACE_BLOCK, 0, st>>>(groups, slots, prefix, n_slots);
+    const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? PSF_OK : cuda_fail(e, "psf_batch_trace launch");
 }
 

@@ -114,10 +114,10 @@ int batch_gemm_smem_bytes(int bn_max);
 // start during that kernel's tail (programmatic dependent launch).
 int launch_batch_step_tc(const StepArgs &args, int bn_max, int grid, cudaStream_t st, bool after_kernel = false);
 int max_fused_grid(int bn_max, int num_sms);
-int launch_batch_state(const GroupDev *groups, SlotDev *slots, int n_slots, cudaStream_t st, bool after_kernel = false);
+int launch_batch_state(const GroupDev *groups, SlotDev *slots, int n_slots, cudaStream_t st);
 // prefix[s] = particles of slots 0..s-1 (occupied slots only); n_slots + 1 entries.
 int launch_batch_trace(const GroupDev *groups, const SlotDev *slots, const long long *prefix, int n_slots, int grid,
-                       bool all_centred, bool faces, cudaStream_t st, bool after_kernel = false);
+                       bool all_centred, bool faces, cudaStream_t st);
 // Put the particles of slots that go on stepping back in brick order where the
 // flow has mixed them.  `round` differs from call to call; `total` is prefix[n_slots].
 // prepare_batch_reorder loads the kernels on the current device, so that no step waits for it.
