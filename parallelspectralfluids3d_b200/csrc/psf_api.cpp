@@ -410,8 +410,8 @@ static int capture_step(psf_ctx *c, int kind, int v, int q, cudaGraph_t *out)
 // 4,096 particles 5.8 us against 8.2 us with a graph per step; 32^3, N = 128,
 // 262,144 particles 17.2 against 20.4; 48^3, N = 256, 1 M particles 75 against
 // 81.  What is left is the reconstruction and the tracer, each of which fills
-// the chip by itself.  RUN_STEPS = 12 keeps a rollout of 50 steps mostly in
-// runs.
+// the chip by itself.  With RUN_STEPS = 12 most of a rollout of 50 steps goes in
+// runs, in a context that has taken RUN_AFTER steps before.
 static int capture_run(psf_ctx *c, int v, int q, cudaGraph_t *out)
 {
     cudaStream_t m = c->stream, s0 = c->side[0], s1 = c->side[1];

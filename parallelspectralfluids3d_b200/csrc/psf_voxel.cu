@@ -62,9 +62,11 @@ int frame_of(const psf_voxel_mesh *m, float res, int mode, Frame *f)
     if (!(res > 0.0f) || !std::isfinite(res)) return fail(PSF_ERR_INVALID, "resolution must be positive and finite");
     // The scan takes 48 coordinates at a time, so that it vectorises: component
     // a of vertex i is coordinate 3 i + a, and lane l of a block of 48 always
-    // meets component l % 3.  psf_voxel_grid of 41,000 vertices 110 -> 33 us from
-    // Python; a whole run does it twice and checks the indices the same way (81,920
-    // triangles into 160^3: 731 -> 616 us, 1,280 into 50^3: 146 -> 136 us).
+    // meets component l % 3.  psf_voxel_grid of 41,000 vertices 113 -> 34 us from
+    // Python; a whole run does it twice (81,920 triangles into 160^3: 764 -> 554 us
+    // warmed, 950 -> 720 with a new mesh; 1,280 into 40^3: 100 -> 98 us).  A
+    // voxeliser's first call is bound by its allocations and the result's page faults
+    // (160^3: 0.98 against 1.0 ms).
     constexpr int LANES = 48;
     float lo[LANES], hi[LANES];
     uint32_t bad = 0;
