@@ -161,15 +161,13 @@ struct psf_batch {
     std::vector<int64_t> slot_units;  // pool units held by each slot
     int64_t bytes = 0;
     std::vector<void *> allocs;
-    // Grouped reads (psf_batch_read_instances): staging for READ_STAGE particles
-    // (or the largest slot), gathered states with a pinned copy, and job table, in
-    // one allocation that read_stage begins.
-    float4 *read_stage = nullptr;
-    double *read_w = nullptr, *read_w_host = nullptr;
-    psf::ReadJob *read_jobs = nullptr;
-    int64_t read_w_cap = 0, read_stage_cap = 0;
-    int64_t read_slots = 0;      // slots asked for before the buffers were made
-    bool reads_singly = false;   // no memory for them
+    // Grouped reads (psf_batch_read_instances): gathered states and job table, which
+    // follow order.staging in its allocation, and the states on the host where they
+    // go to several places.
+    double *read_w = nullptr;
+    psf::ReadJob *read_jobs = nullptr;  // null: no memory for grouped reads
+    int64_t read_w_cap = 0, stage_cap = 0;  // particles order.staging holds
+    std::vector<double> read_w_host;
     // Reads of slots that the queued steps do not touch (psf::batch_read_frozen):
     // a second stream and pinned host buffers for one slot's particles.
     cudaStream_t side = nullptr;
@@ -183,8 +181,6 @@ struct psf_batch {
     {
         drop_graph();
         for (void *p : allocs) cudaFree(p);
-        cudaFree(read_stage);
-        if (read_w_host) cudaFreeHost(read_w_host);
         if (rd_parts) cudaFreeHost(rd_parts);
         if (rd_perm) cudaFreeHost(rd_perm);
         if (side) cudaStreamDestroy(side);
@@ -432,47 +428,33 @@ int check_device_error(psf_batch *B)
     return PSF_OK;
 }
 
-// Particles the staging buffer of grouped reads holds (64 MB), unless one slot
-// holds more.
-constexpr int64_t READ_STAGE = 4 << 20;
-// Their buffers are made once, for the largest read, by the read with which so
-// many slots have been asked for: 0.5 to 2 ms, and a grouped read is 9 to 16 us a
-// slot shorter (two slots 53 -> 44 us, 64 slots of 4,096 particles 890 -> 124,
-// 96 of 65,536 3.48 -> 1.88 ms).  A batch that is read less than that pays nothing.
-constexpr int64_t READ_AFTER = 128;
+// Particles that a grouped read gathers at a time (16 MB), unless one slot holds
+// more.
+constexpr int64_t READ_STAGE = 1 << 20;
 
-// Whether a read of n slots goes through the buffers of grouped reads; not where
-// memory for them is short.
-bool group_read(psf_batch *B, int64_t n, int64_t n_w)
+// The ordering scratch's staging buffer, which holds the largest slot, and with it
+// the buffers of grouped reads: several slots in staging, the states of all slots
+// and a job for each.  They are made with the batch because a first read that made
+// them took 0.5 to 2 ms longer.  The last of a batch's buffers: where there is no
+// memory for them, staging for one slot, and reads go slot by slot.
+int alloc_staging(psf_batch *B)
 {
-    const int64_t jobs = B->n_slots();
-    if (n < 2 || n > jobs || B->reads_singly) return false;
-    if (!B->read_jobs) {
-        B->read_slots += n;
-        if (B->read_slots < READ_AFTER) return false;
-        int64_t rows = 0;
-        for (const HostGroup &G : B->groups) rows += (int64_t)G.cap * G.N;
-        const int64_t stage = std::max(std::min(B->pool_cap, READ_STAGE), B->pmax_all);
-        const size_t at_w = (size_t)stage * sizeof(float4), at_jobs = at_w + (size_t)rows * sizeof(double);
-        const size_t bytes = at_jobs + (size_t)jobs * sizeof(psf::ReadJob);
-        unsigned char *p = nullptr;
-        double *host = nullptr;
-        if (cudaMalloc(&p, bytes) != cudaSuccess ||
-            cudaHostAlloc((void **)&host, (size_t)rows * 8, cudaHostAllocDefault) != cudaSuccess) {
-            cudaGetLastError();
-            cudaFree(p);
-            B->reads_singly = true;
-            return false;
-        }
-        B->read_stage = reinterpret_cast<float4 *>(p);
-        B->read_w = reinterpret_cast<double *>(p + at_w);
-        B->read_jobs = reinterpret_cast<psf::ReadJob *>(p + at_jobs);
-        B->read_w_host = host;
-        B->read_w_cap = rows;
-        B->read_stage_cap = stage;
-        B->bytes += (int64_t)bytes;
+    int64_t rows = 0;
+    for (const HostGroup &G : B->groups) rows += (int64_t)G.cap * G.N;
+    const int64_t stage = std::max(std::min(B->pool_cap, READ_STAGE), B->pmax_all);
+    const size_t at_w = (size_t)stage * sizeof(float4), at_jobs = at_w + (size_t)rows * sizeof(double);
+    unsigned char *p = nullptr;
+    B->stage_cap = B->pmax_all;
+    if (B->alloc(&p, at_jobs + B->slots.size() * sizeof(psf::ReadJob)) != PSF_OK) {
+        cudaGetLastError();
+        return B->alloc(&B->order.staging, (size_t)B->pmax_all);
     }
-    return n_w <= B->read_w_cap;
+    B->order.staging = reinterpret_cast<float4 *>(p);
+    B->read_w = reinterpret_cast<double *>(p + at_w);
+    B->read_jobs = reinterpret_cast<psf::ReadJob *>(p + at_jobs);
+    B->read_w_cap = rows;
+    B->stage_cap = stage;
+    return PSF_OK;
 }
 
 // Where the host memory that one copy may cover ends, starting from a host
@@ -508,7 +490,7 @@ struct CopyRange {
         kind = REGISTERED;
         end = (uintptr_t)start + size;
     }
-    // Whether the buffer at p, which follows what is covered so far, is covered too.
+    // Whether the buffer at p, which begins or follows what is covered so far, is covered too.
     bool covers(const void *p, size_t bytes) const
     {
         if (kind == REGISTERED) return (uintptr_t)p + bytes <= end;
@@ -837,12 +819,13 @@ int psf_batch_create(const psf_batch_config *cfg, int device, psf_batch **out)
         psf::OrderBufs &o = B->order;
         size_t tmp = 0;
         unsigned char *temp = nullptr;
-        if ((rc = psf::sort_particles_temp_bytes(B->pmax_all, &tmp)) || (rc = B->alloc(&o.staging, B->pmax_all)) ||
+        if ((rc = psf::sort_particles_temp_bytes(B->pmax_all, &tmp)) ||
             (rc = B->alloc(&o.keys_in, B->pmax_all)) || (rc = B->alloc(&o.keys_out, B->pmax_all)) ||
             (rc = B->alloc(&o.idx_in, B->pmax_all)) || (rc = B->alloc(&temp, tmp)))
             return bail(rc);
         o.temp = temp;
         o.temp_bytes = tmp;
+        if ((rc = alloc_staging(B)) != PSF_OK) return bail(rc);
     }
     fill_gemm_args(B);
     if ((rc = upload_tables(B)) != PSF_OK || (rc = upload_prefix(B)) != PSF_OK) return bail(rc);
@@ -1060,34 +1043,44 @@ int psf_batch_read_instances(psf_batch *B, int32_t n, const int32_t *basis, cons
         j.n_parts = xyzw[i] ? (int)s.n_particles : 0;
         n_w += j.n_w;
     }
-    if (!group_read(B, n, n_w)) return read_one_by_one(B, jobs, w, xyzw);
+    if (n < 2 || n > B->n_slots() || !B->read_jobs || n_w > B->read_w_cap) return read_one_by_one(B, jobs, w, xyzw);
     // Groups of slots that fill the staging buffer: [first, last).
     std::vector<std::pair<int32_t, int32_t>> groups;
+    // The states go to the caller in one copy where the caller's buffers follow one
+    // another in page-locked memory, else through host memory of the batch.
+    bool one_w = true;
+    double *w_to = nullptr;
     try {
         for (int32_t i = 0; i < n;) {
             const int32_t first = i;
             int64_t at = 0;
-            for (; i < n && at + jobs[(size_t)i].n_parts <= B->read_stage_cap; ++i) {
+            for (; i < n && at + jobs[(size_t)i].n_parts <= B->stage_cap; ++i) {
                 jobs[(size_t)i].stage = at;
                 at += jobs[(size_t)i].n_parts;
             }
             groups.emplace_back(first, i);
         }
+        int32_t first = 0;
+        while (first < n && jobs[(size_t)first].n_w == 0) ++first;
+        for (int32_t i = first; i < n && one_w; ++i)
+            one_w = jobs[(size_t)i].n_w == 0 || w[i] == w[first] + jobs[(size_t)i].w_at;
+        if (n_w > 0 && one_w) {
+            const CopyRange range(w[first]);
+            one_w = range.kind == CopyRange::REGISTERED && range.covers(w[first], (size_t)n_w * 8);
+        }
+        if (!one_w && (int64_t)B->read_w_host.size() < n_w) B->read_w_host.resize((size_t)B->read_w_cap);
+        w_to = n_w > 0 && one_w ? w[first] : B->read_w_host.data();
     } catch (const std::bad_alloc &) {
         return fail(PSF_ERR_NOMEM, "host allocation failed");
     }
     cudaStream_t st = B->stream;
     PSF_CUDA(cudaMemcpyAsync(B->read_jobs, jobs.data(), jobs.size() * sizeof(psf::ReadJob), cudaMemcpyHostToDevice, st));
-    if (n_w > 0) {
-        PSF_CHECK(psf::launch_batch_gather_states(B->read_jobs, n, B->read_w, st));
-        PSF_CUDA(cudaMemcpyAsync(B->read_w_host, B->read_w, (size_t)n_w * 8, cudaMemcpyDeviceToHost, st));
-    }
     for (const auto &g : groups) {
         int most = 0;
         for (int32_t i = g.first; i < g.second; ++i) most = std::max(most, jobs[(size_t)i].n_parts);
         if (most == 0) continue;
         PSF_CHECK(psf::launch_batch_unorder(B->read_jobs + g.first, g.second - g.first, most, B->pool_parts,
-                                            B->pool_perm, B->read_stage, st));
+                                            B->pool_perm, B->order.staging, st));
         // One copy for slots whose host buffers follow one another in one piece of memory.
         for (int32_t i = g.first; i < g.second;) {
             const int32_t first = i;
@@ -1104,14 +1097,18 @@ int psf_batch_read_instances(psf_batch *B, int32_t n, const int32_t *basis, cons
                     ++i;
                 }
             }
-            PSF_CUDA(cudaMemcpyAsync(xyzw[first], B->read_stage + jobs[(size_t)first].stage, (size_t)count * 16,
+            PSF_CUDA(cudaMemcpyAsync(xyzw[first], B->order.staging + jobs[(size_t)first].stage, (size_t)count * 16,
                                      cudaMemcpyDeviceToHost, st));
         }
     }
+    if (n_w > 0) {
+        PSF_CHECK(psf::launch_batch_gather_states(B->read_jobs, n, B->read_w, st));
+        PSF_CUDA(cudaMemcpyAsync(w_to, B->read_w, (size_t)n_w * 8, cudaMemcpyDeviceToHost, st));
+    }
     PSF_CHECK(check_device_error(B));
-    for (int32_t i = 0; i < n; ++i)
+    for (int32_t i = 0; i < n && !one_w; ++i)
         if (jobs[(size_t)i].n_w)
-            std::memcpy(w[i], B->read_w_host + jobs[(size_t)i].w_at, (size_t)jobs[(size_t)i].n_w * 8);
+            std::memcpy(w[i], w_to + jobs[(size_t)i].w_at, (size_t)jobs[(size_t)i].n_w * 8);
     return PSF_OK;
 }
 

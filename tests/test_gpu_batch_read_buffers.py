@@ -1,4 +1,4 @@
-"""Grouped read-back makes its buffers once, and not for a batch that is hardly read."""
+"""Grouped read-back of every size, and states to one place or several, from buffers made with the batch."""
 import numpy as np
 import pytest
 
@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 # Slots of two bases with counts below the staging, above it, and one slot that fills it.
 @pytest.mark.parametrize("counts", [(300, 0, 257, 1, 4096, 33, 512, 2), (1300000, 700, 1500000, 1400000), (40, 5000000)])
-def test_buffers_made_once(small_bases, counts):
+def test_reads_of_every_size(small_bases, counts):
     bases = [small_bases["box576"], small_bases["sphere12x10x9"]]
     params = L.make_params(dt=0.01, precision=L.PSF_PRECISION_BF16X2)
     n = len(counts)
@@ -41,8 +41,17 @@ def test_buffers_made_once(small_bases, counts):
             for k in range(n):
                 assert np.array_equal(w[k], want[k][0] if k < m else np.full(len(w[k]), -7.0))
                 assert np.array_equal(p[k], want[k][1]) if k < m else np.all(p[k] == -7.0)
-        assert sizes[1] == sizes[0]  # a first read of two slots makes none
-        assert len(set(sizes)) == 2 and sizes == sorted(sizes)
+        assert len(set(sizes)) == 1  # no read allocates
+        # States that follow one another in page-locked memory, all or some of them wanted.
+        import torch
+        row = torch.empty(sum(len(x[0]) for x in want), dtype=torch.float64, pin_memory=True).numpy()
+        ends = np.cumsum([len(x[0]) for x in want])
+        w = [row[e - len(x[0]):e] for x, e in zip(want, ends)]
+        for left_out in (None, 0, n - 1):
+            row[:] = -7.0
+            L.check(read(bt, where, [None if k == left_out else a for k, a in enumerate(w)], [None] * n))
+            for k in range(n):
+                assert np.array_equal(w[k], want[k][0]) if k != left_out else np.all(w[k] == -7.0)
         # The same slot more often than there are slots.
         twice = [where[0]] * (2 * bt.slots[0] + 1)
         q = [np.empty((counts[0], 4), np.float32) for _ in twice]

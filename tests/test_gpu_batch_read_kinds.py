@@ -34,7 +34,7 @@ def test_partly_registered(small_bases, locked):
                 bt.set_instance(0, s, initial_coefficients(b.n_modes, s), params, initial_particles(b, COUNT, s))
             bt.step(2)
             want = [bt.get_particles(0, s) for s in range(6)]
-            for _ in range(24):  # single reads at first, then grouped ones
+            for _ in range(3):
                 flat[:] = -7.0
                 w = [np.zeros(b.n_modes) for _ in range(6)]
                 L.check(read(bt, [(0, s) for s in range(6)], w, p))
