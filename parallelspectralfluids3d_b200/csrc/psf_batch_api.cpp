@@ -638,9 +638,10 @@ int launch_step(psf_batch *B, cudaStream_t st, bool after_kernel)
 // 184 us).  Nor the state update, whose blocks hold up the contraction's end
 // (67.5 us for 40 of N = 200).  Capturing it costs 30 us more than the graph of
 // one step, so a batch that has taken and is asked for fewer than RUN_PAYS steps
-// does without (a new batch's first 8 steps: 329 us, with it 360).
+// does without (a new batch's first 8 steps: 329 us, with it 360; 16: 492 and 510;
+// 50: 1,206 and 1,141).
 constexpr int RUN_STEPS = 8;
-constexpr int RUN_PAYS = 2 * RUN_STEPS;
+constexpr int RUN_PAYS = 3 * RUN_STEPS;
 
 // Steps between two looks at the particles' order (psf_batch_reorder).
 constexpr int ORDER_EVERY = 64;
