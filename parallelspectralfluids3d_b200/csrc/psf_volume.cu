@@ -291,8 +291,9 @@ __device__ __forceinline__ float len3(float x, float y, float z)
 // others waited) and 3.1 ms for a lane that switches between its march and its
 // shadow ray (long rays then walk thousands of samples alone).  2 M particles,
 // normal cloud: 1.55 against 11.6 ms; 100,000 in 128^3, 640 x 360: 3.2 against
-// 22.7 ms.  It is bound by issue (80 % of the slots, 17.6 lanes per
-// instruction) with the occupancy words and pairs in L1 and L2.  One
+// 22.7 ms.  It is bound by issue (16.8 M particles, normal cloud:
+// 76 % of the slots, 20.5 lanes per instruction) with the occupancy words and
+// pairs in L1 and L2.  One
 // occupancy look-up at a time took 2.7 ms at the first size (its load latency
 // stood between any two steps); POOL = 512 or 8 blocks per SM changed nothing.
 constexpr int RENDER_THREADS = 128;

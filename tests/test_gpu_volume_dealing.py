@@ -15,8 +15,8 @@ pytestmark = pytest.mark.gpu
     (48, 45, 31, 12000, 1.0, (0.8, -0.6, 0.9)),    # most cells: walks without look-ups, and back
     (33, 31, 45, 2500, 1.0, (0.8, -0.6, 0.9)),     # fewer than half, R above 32
     (32, 31, 45, 60, 1.0, (0.8, -0.6, 0.9)),       # few cells of eight steps
-    (16, 131, 120, 150000, 0.1, (0.01, 0.02, 0.0)),  # filled and opaque, camera inside: larger hands
-    (16, 131, 120, 150000, 0.1, (0.1, -0.05, 0.12)), # ... and outside
+    (16, 161, 131, 150000, 0.1, (0.01, 0.02, 0.0)),  # filled and opaque, camera inside: larger hands
+    (16, 161, 131, 150000, 0.1, (0.1, -0.05, 0.12)), # ... and outside
     (16, 19, 13, 30000, 1.0, (0.1, 0.2, 0.1)),        # filled, long shadow rays
 ])
 def test_dealing(res, width, height, count, size, eye):
