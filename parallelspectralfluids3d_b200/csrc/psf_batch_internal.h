@@ -66,6 +66,10 @@ struct StepArgs {
     int n_slots;
 };
 
+// SlotDev::stepped, else 0: the slot advanced, and with it a flow that carries most
+// particles out of their half-cell in an RK4 step.
+constexpr int STEPPED = 1, STEPPED_FAST = 2;
+
 // Per-slot parameters and counters, in device memory.
 struct SlotDev {
     int active;
@@ -77,13 +81,13 @@ struct SlotDev {
     double dt;
     double visc_signed;
     float lifetime;
-    float pad0;
+    float fast_above;         // |w|^2 above which the slot's flow is fast (FAST_STEP)
     unsigned long long seed;
     unsigned long long step;  // steps taken since the slot was set (device counter)
     long long n_particles;
     long long poff;           // first particle of the slot in the particle pool
     unsigned long long target;  // stop after this many steps (0: no limit)
-    int stepped;              // 1 if the slot advanced in the current step (set by the state kernel)
+    int stepped;              // STEPPED or STEPPED_FAST if the slot advanced in the current step (set by the state kernel)
     int mixed;                // round of launch_batch_reorder in which the slot was out of order
 };
 
