@@ -596,7 +596,8 @@ __global__ void psf_batch_unorder(const ReadJob *__restrict__ jobs, const float4
 // half-cell or whose life is over, and takes 32 of them at once: otherwise one
 // such lane holds the other 31 for up to three more gathers.  Slots whose flow
 // carries most particles out of their half-cell (FAST_STEP) go straight through
-// after the others.  16 x 262,144
+// after the others, and so do all where no thread has two particles (65,536 on
+// 16^3 16.7 against 18.2 us a step; 131,072, beyond the grid, 19.6 either way).  16 x 262,144
 // particles on the 32^3 box with a sphere, RK4: 107 against 126 us at 0.03 voxel
 // per step, 136 against 141 at 0.12, 96 against 98 at 0.001; RK1 70 either way.
 // Where faces are stored once (few particles per voxel) a warp's particles lie
@@ -665,12 +666,12 @@ __device__ __forceinline__ int slot_of_particle(const long long *pre, int n_slot
     return lo;
 }
 
-// The particles of fast slots, each straight through: hardly one stays in its
-// half-cell, and trying it there first cost up to 37 % (16 x 262,144, RK4, 0.9 voxel
-// per step: 376 against 275 us).  A function of its own: inlined, its registers cost
-// the slow slots' loop 5 %.
-__device__ __noinline__ void trace_fast(const GroupDev *__restrict__ groups, const SlotDev *__restrict__ slots,
-                                        const long long *pre, int n_slots, long long total)
+// The particles of slots that stepped in one of the ways from `least` on, each
+// straight through.  In fast slots hardly one stays in its half-cell, and trying it
+// there first cost up to 37 % (16 x 262,144, RK4, 0.9 voxel per step: 376 against 275
+// us).  A function of its own: inlined, its registers cost the slow slots' loop 5 %.
+__device__ __noinline__ void trace_straight(const GroupDev *__restrict__ groups, const SlotDev *__restrict__ slots,
+                                            const long long *pre, int n_slots, long long total, int least)
 {
     int cur = -1;
     TraceSlot t;
@@ -679,7 +680,7 @@ __device__ __noinline__ void trace_fast(const GroupDev *__restrict__ groups, con
         if (cur < 0 || gi >= pre[cur + 1]) {
             cur = slot_of_particle(pre, n_slots, cur, gi);
             t.load(groups, slots[cur], pre[cur]);
-            t.live = slots[cur].stepped == STEPPED_FAST;
+            t.live = slots[cur].stepped >= least;
         }
         if (t.live) t.advance<CentredBox<PairField>>(t.base + (size_t)gi);
     }
@@ -711,6 +712,12 @@ __global__ void __launch_bounds__(TRACE_BLOCK, 5) psf_batch_trace(const GroupDev
     uint32_t *aa = aside_at[ASIDE ? warp : 0];
     const long long total = pre[n_slots];
     const long long stride = (long long)gridDim.x * blockDim.x;
+    if constexpr (ASIDE) {
+        if (total <= stride) {  // no second particle to put with those put aside
+            trace_straight(groups, slots, pre, n_slots, total, STEPPED);
+            return;
+        }
+    }
     // Parameters of the slot the thread is in, reloaded only when it changes.
     int cur = -1, waiting = 0;
     TraceSlot t;
@@ -757,7 +764,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK, 5) psf_batch_trace(const GroupDev
     if constexpr (ASIDE) {
         __syncwarp();
         if (lane < waiting) trace_later(groups, slots[as[lane]], aa[lane]);
-        if (any_fast) trace_fast(groups, slots, pre, n_slots, total);
+        if (any_fast) trace_straight(groups, slots, pre, n_slots, total, STEPPED_FAST);
     }
 }
 

@@ -5,6 +5,7 @@ import pytest
 from parallelspectralfluids3d_b200 import _lib as L
 from parallelspectralfluids3d_b200.batch import Batch
 from parallelspectralfluids3d_b200.fixture import initial_coefficients, initial_particles
+from test_gpu_particle_order import toy_basis
 
 pytestmark = pytest.mark.gpu
 
@@ -36,3 +37,32 @@ def test_fast_slots(small_bases, integrator, fused):
         assert np.array_equal(x[1], y[1], equal_nan=True)
     moved = [np.isfinite(p).any() for _, p in out[0]]
     assert all(moved)
+
+
+@pytest.mark.parametrize("integrator", [L.PSF_RK1, L.PSF_RK4])
+@pytest.mark.parametrize("count", [30000, 60000])  # three slots: below and above a particle per thread of the grid
+def test_slow_and_fast_with_lists(integrator, count):
+    b = toy_basis((64, 48, 48))
+    dt = 0.01
+    params = L.make_params(dt=dt, integrator=integrator, lifetime=6.0, seed=2, precision=L.PSF_PRECISION_BF16X2)
+    rng = np.random.default_rng(count)
+    size = np.asarray(b.aabb_max) - b.aabb_min
+    start = []
+    for s in range(3):
+        p = np.full((count - 7 * s, 4), np.inf, np.float32)
+        p[:, :3] = b.aabb_min + size * rng.random((len(p), 3), dtype=np.float32)
+        p[::9, 3] = np.arange(len(p[::9])) % 8
+        start.append(p)
+    out = []
+    for capacity in (3 * b.n_voxels, count):  # pairs, faces once
+        with Batch([b], 3, capacity, autotune=False, particle_pool=3 * count + 1024) as bt:
+            for s, step in enumerate((0.02, 0.6, 0.119)):
+                w0 = np.array([1.0, -2.0, 0.5])
+                w0 *= step * b.h * np.sqrt(b.n_active) / (dt * np.linalg.norm(w0))
+                bt.set_instance(0, s, w0, params, start[s])
+            bt.step(10)
+            out.append([bt.get_particles(0, s) for s in range(3)])
+    for x, y in zip(*out):
+        assert np.array_equal(x, y)
+    moved = np.abs(out[0][1][:, :3] - start[1][:, :3]).max(axis=1) / b.h
+    assert np.median(moved) > 1.0
